@@ -20,6 +20,7 @@
 // oracle at 1e-12 relative L2 per field).
 #pragma once
 #include "enl_fast.cuh"
+#include "enl_triple.cuh"
 
 namespace enl {
 
@@ -77,38 +78,79 @@ __device__ __forceinline__ int sensor_line_fast(const double r[5], double ep) {
   return tag;
 }
 
-// FP64 planes of a 38 x 14 halo tile (rows of kBW64 doubles): u and v at
-// every position, the half fluxes F_0..4 / 2 on the 8 interior rows and
-// G_0..4 / 2 on the 32 interior columns (rows of 32).
-constexpr int kBW64 = 38, kBH64 = 14;
-constexpr int kPos64 = kBW64 * kBH64;       // 532
-constexpr int kPl64F = 8 * kBW64;           // 304
-constexpr int kPl64G = kBH64 * 32;          // 448
-constexpr int kPl64OffV = kPos64, kPl64OffF = 2 * kPos64, kPl64OffG = kPl64OffF + 5 * kPl64F;
-constexpr int kPl64Elems = kPl64OffG + 5 * kPl64G;  // 4824 doubles
+// FP64 planes of a 38 x (TH + 6) halo tile (rows of kBW64 doubles; TH = 8 in
+// the batched engine): u and v at every position, the half fluxes F_0..4 / 2
+// on the TH interior rows and G_0..4 / 2 on the 32 interior columns (rows of
+// 32).
+constexpr int kBW64 = 38;
+template <int TH>
+struct Geo64 {
+  static constexpr int BH = TH + 6;
+  static constexpr int Pos = kBW64 * BH;
+  static constexpr int PF = TH * kBW64, PG = BH * 32;
+  static constexpr int OffV = Pos, OffF = 2 * Pos, OffG = OffF + 5 * PF;
+  static constexpr int Elems = OffG + 5 * PG;
+};
 
-// Accessor of one cell: the staged tile (7 fields, planes of kPos64) and the
+// Accessor of one cell: the staged tile (7 fields, planes of Pos) and the
 // planes, centred on the cell.
+template <int TH>
 struct SAcc64P {
+  using G = Geo64<TH>;
   const double* t;
   const double* pl;
   int c;       // (cy + 3) * kBW64 + cx + 3
   int cf, cg;  // cy * kBW64 + cx + 3 in the F planes, (cy + 3) * 32 + cx in the G planes
-  __device__ double w(int k, int di, int dj) const { return t[k * kPos64 + c + dj * kBW64 + di]; }
-  __device__ double p(int di, int dj) const { return t[5 * kPos64 + c + dj * kBW64 + di]; }
-  __device__ double t_(int di, int dj) const { return t[6 * kPos64 + c + dj * kBW64 + di]; }
+  __device__ double w(int k, int di, int dj) const { return t[k * G::Pos + c + dj * kBW64 + di]; }
+  __device__ double p(int di, int dj) const { return t[5 * G::Pos + c + dj * kBW64 + di]; }
+  __device__ double t_(int di, int dj) const { return t[6 * G::Pos + c + dj * kBW64 + di]; }
   __device__ double u(int di, int dj) const { return pl[c + dj * kBW64 + di]; }
-  __device__ double v(int di, int dj) const { return pl[kPl64OffV + c + dj * kBW64 + di]; }
-  __device__ double fx(int k, int di) const { return pl[kPl64OffF + k * kPl64F + cf + di]; }
-  __device__ double gy(int k, int dj) const { return pl[kPl64OffG + k * kPl64G + cg + dj * 32]; }
+  __device__ double v(int di, int dj) const { return pl[G::OffV + c + dj * kBW64 + di]; }
+  __device__ double fx(int k, int di) const { return pl[G::OffF + k * G::PF + cf + di]; }
+  __device__ double gy(int k, int dj) const { return pl[G::OffG + k * G::PG + cg + dj * 32]; }
 };
-__device__ __forceinline__ SAcc64P acc64p(const double* t, const double* pl, int cx, int cy) {
-  return SAcc64P{t, pl, (cy + 3) * kBW64 + cx + 3, cy * kBW64 + cx + 3, (cy + 3) * 32 + cx};
+template <int TH>
+__device__ __forceinline__ SAcc64P<TH> acc64p(const double* t, const double* pl, int cx, int cy) {
+  return SAcc64P<TH>{t, pl, (cy + 3) * kBW64 + cx + 3, cy * kBW64 + cx + 3, (cy + 3) * 32 + cx};
+}
+
+// The planes of a tile of w x h cells from its staged box, by the whole block
+// of 256 threads (no barrier inside).  One seeded reciprocal of rho per halo
+// position; the flux planes hold half fluxes, formed from u/2, v/2 and p/2
+// (halving is exact, so each is F/2 or G/2 of the same double).  The
+// positions past a multiple of 256 fall on the last warp, not on warp 0, which
+// also stages the engine's next tile.
+template <int TH>
+__device__ __forceinline__ void build_planes64(const double* tile, double* pl, int w, int h) {
+  using G = Geo64<TH>;
+  for (int e = 255 - (int)threadIdx.x; e < G::Pos; e += 256) {
+    const int row = e / kBW64, col = e - row * kBW64;
+    if (row >= h + 6 || col >= w + 6) continue;  // beyond a ragged tile
+    const double ir = rcp64(tile[e]);
+    const double u = tile[G::Pos + e] * ir, v = tile[2 * G::Pos + e] * ir;
+    const double hp = 0.5 * tile[5 * G::Pos + e];
+    pl[e] = u;
+    pl[G::OffV + e] = v;
+    if (row >= 3 && row < 3 + TH) {
+      const double hu = 0.5 * u;
+#pragma unroll
+      for (int k = 0; k < 5; ++k)
+        pl[G::OffF + k * G::PF + (row - 3) * kBW64 + col] =
+            k == 1 ? fma(hu, tile[G::Pos + e], hp) : hu * tile[k * G::Pos + e];
+    }
+    if (col >= 3 && col < 3 + 32) {
+      const double hv = 0.5 * v;
+#pragma unroll
+      for (int k = 0; k < 5; ++k)
+        pl[G::OffG + k * G::PG + row * 32 + (col - 3)] =
+            k == 2 ? fma(hv, tile[2 * G::Pos + e], hp) : hv * tile[k * G::Pos + e];
+    }
+  }
 }
 
 // Switch of one cell (SCHEME as in enl_physics.cuh).
-template <int SCHEME>
-__device__ __forceinline__ int switch64(const SAcc64P& A, const RhsConst& P) {
+template <int SCHEME, int TH>
+__device__ __forceinline__ int switch64(const SAcc64P<TH>& A, const RhsConst& P) {
   if (SCHEME == kWeno) return 1;
   if (SCHEME == kDrp) return 0;
   if (P.level != 0) return 1;
@@ -123,7 +165,8 @@ __device__ __forceinline__ int switch64(const SAcc64P& A, const RhsConst& P) {
 
 // Viscous, entropy-production and relaxation sources H1..H4
 // (rhs_hybrid_high_llf.m4:161-237) from the planes.
-__device__ __forceinline__ void sources64(const SAcc64P& A, const RhsConst& P, double H[5]) {
+template <int TH>
+__device__ __forceinline__ void sources64(const SAcc64P<TH>& A, const RhsConst& P, double H[5]) {
   const double c43 = Lit::c4_3, c23 = Lit::c2_3;
   double u[3][3], v[3][3];
 #pragma unroll
@@ -174,174 +217,119 @@ __device__ __forceinline__ void sources64(const SAcc64P& A, const RhsConst& P, d
   H[4] = (rho * P.inv_tau_n) * (Tc - T_n);
 }
 
-// WENO5 reconstruction (the formulas of weno5 in enl_physics.cuh) from its
-// five inputs and the squares of its three second differences tt0..tt2
-// (S0 = c,d,e; S1 = b,c,d; S2 = a,b,c), arranged for the FP64 pipe:
-//   * the weights omega_k = (d_k / q_k) / sum_j (d_j / q_j) do not change
-//     when every q_k is multiplied by the same number, so with
-//     q_k = (13/12 t_k^2 + s_k^2 / 4 + eps)^2 the routine uses 16 q_k =
-//     (13/3 t_k^2 + s_k^2 + 4 eps)^2, formed by two fused multiply-adds and
-//     a square;
-//   * omega_k f_k / 6 = P_k (d_k f_k / 6) / sum_j d_j P_j with P_k the product
-//     of the other two q: the linear weights d_k and the 1/6 go into the
-//     candidate polynomials' coefficients (compile-time constants), and the
-//     normalisation is one seeded reciprocal.
-// The result agrees with weno5 to rounding.
-template <bool PLUS>
-__device__ __forceinline__ double weno5q(double a, double b, double c, double d, double e, double tt0, double tt1,
-                                         double tt2) {
-  constexpr double k4 = 4.0 * Lit::c13_12;        // exact
-  constexpr double eps4 = 4.0 * Lit::weno_eps;    // exact
-  const double s0 = fma(3.0, c, fma(-4.0, d, e)), s1 = b - d, s2 = fma(3.0, c, fma(-4.0, b, a));
-  double q0 = fma(k4, tt0, fma(s0, s0, eps4));
-  double q1 = fma(k4, tt1, fma(s1, s1, eps4));
-  double q2 = fma(k4, tt2, fma(s2, s2, eps4));
-  q0 *= q0;
-  q1 *= q1;
-  q2 *= q2;
-  constexpr double d0 = PLUS ? Lit::c0_3 : Lit::c0_1;
-  constexpr double d1 = Lit::c0_6;
-  constexpr double d2 = PLUS ? Lit::c0_1 : Lit::c0_3;
-  constexpr double w0 = d0 * Lit::c1_6, w1 = d1 * Lit::c1_6, w2 = d2 * Lit::c1_6;
-  const double P0 = q1 * q2, P1 = q0 * q2, P2 = q0 * q1;
-  const double den = fma(d0, P0, fma(d1, P1, d2 * P2));
-  double g0, g1, g2;  // d_k f_k / 6
-  if (PLUS) {
-    g0 = fma(2.0 * w0, c, fma(5.0 * w0, d, -w0 * e));
-    g1 = fma(-w1, b, fma(5.0 * w1, c, (2.0 * w1) * d));
-    g2 = fma(2.0 * w2, a, fma(-7.0 * w2, b, (11.0 * w2) * c));
-  } else {
-    g0 = fma(11.0 * w0, c, fma(-7.0 * w0, d, (2.0 * w0) * e));
-    g1 = fma(2.0 * w1, b, fma(5.0 * w1, c, -w1 * d));
-    g2 = fma(-w2, a, fma(5.0 * w2, b, (2.0 * w2) * c));
-  }
-  const double num = fma(P0, g0, fma(P1, g1, P2 * g2));
-  return num * rcp64(den);
-}
-
-// The two WENO5 reconstructions of one sign along one direction of a cell:
-// x[0..5] are the split fluxes at offsets -3..2; lo is the reconstruction
-// from x[0..4], hi from x[1..5].  The two stencils share two of their three
-// second differences and those differences' squares.
-template <bool PLUS>
-__device__ __forceinline__ void weno5_pair(const double x[6], double& lo, double& hi) {
-  double tt[4];
+// Flux part of the five fields of a DRP cell, dF/dx + dG/dy (Tam-Webb,
+// rhs_hybrid_high_llf.m4:258-268).  The planes hold half fluxes: the
+// coefficients are doubled (exactly).
+template <int TH>
+__device__ __forceinline__ void drp_flux64(const SAcc64P<TH>& A, const RhsConst& P, double D[5]) {
 #pragma unroll
-  for (int j = 0; j < 4; ++j) {
-    const double t = fma(-2.0, x[j + 1], x[j]) + x[j + 2];
-    tt[j] = t * t;
-  }
-  lo = weno5q<PLUS>(x[0], x[1], x[2], x[3], x[4], tt[2], tt[1], tt[0]);
-  hi = weno5q<PLUS>(x[1], x[2], x[3], x[4], x[5], tt[3], tt[2], tt[1]);
-}
-
-template <bool PLUS>
-__device__ __forceinline__ double weno3r(double b, double c, double d) {
-  double e0 = d - c, e1 = c - b;
-  double q0 = fma(e0, e0, Lit::weno_eps), q1 = fma(e1, e1, Lit::weno_eps);
-  q0 *= q0;
-  q1 *= q1;
-  const double z0 = PLUS ? Lit::c2_3 : Lit::c1_3;
-  const double z1 = PLUS ? Lit::c1_3 : Lit::c2_3;
-  double n0 = z0 * q1, n1 = z1 * q0;
-  double f0 = PLUS ? (c + d) : fma(3.0, c, -d);
-  double f1 = PLUS ? fma(3.0, c, -b) : (b + c);
-  return (0.5 * fma(n0, f0, n1 * f1)) * rcp64(n0 + n1);
-}
-
-// LLF-split WENO derivative of field k plus its source hk (out of line: one
-// copy of the code for the five fields).
-// The planes hold half fluxes F/2, G/2, and ha, hb are half the split
-// speeds: fma(ha, w, F/2) is 0.5 fma(af, w, F) exactly (halving is exact),
-// one multiplication fewer per split flux.
-template <int ORDER>
-__device__ __noinline__ double weno_field64(const SAcc64P A, const RhsConst& P, int k, double ha, double hb,
-                                            double hk) {
-  double fp[7], fm[7], gp[7], gm[7];
+  for (int k = 0; k < 5; ++k) {
+    double fx = 0.0, gy = 0.0;
 #pragma unroll
-  for (int q = 0; q < 7; ++q) {
-    const double wx = A.w(k, q - 3, 0), wy = A.w(k, 0, q - 3);
-    const double Fh = A.fx(k, q - 3), Gh = A.gy(k, q - 3);
-    fp[q] = fma(ha, wx, Fh);
-    fm[q] = fma(-ha, wx, Fh);
-    gp[q] = fma(hb, wy, Gh);
-    gm[q] = fma(-hb, wy, Gh);
-  }
-  double dfx, dgy;
-  if (ORDER == 5) {
-    double fpl, fph, fml, fmh, gpl, gph, gml, gmh;
-    weno5_pair<true>(fp, fpl, fph);
-    weno5_pair<false>(fm + 1, fml, fmh);
-    weno5_pair<true>(gp, gpl, gph);
-    weno5_pair<false>(gm + 1, gml, gmh);
-    dfx = ((fpl + fml) - fph) - fmh;
-    dgy = ((gpl + gml) - gph) - gmh;
-  } else {
-    dfx = ((weno3r<true>(fp[1], fp[2], fp[3]) + weno3r<false>(fm[2], fm[3], fm[4])) -
-           weno3r<true>(fp[2], fp[3], fp[4])) -
-          weno3r<false>(fm[3], fm[4], fm[5]);
-    dgy = ((weno3r<true>(gp[1], gp[2], gp[3]) + weno3r<false>(gm[2], gm[3], gm[4])) -
-           weno3r<true>(gp[2], gp[3], gp[4])) -
-          weno3r<false>(gm[3], gm[4], gm[5]);
-  }
-  return fma(dfx, P.inv_dx0, fma(dgy, P.inv_dx1, hk));
-}
-
-// KK[0..4] of the cell given the switch (H[0] holds the source H0).
-template <int ORDER, bool LLF>
-__device__ __forceinline__ void fluxes64(const SAcc64P& A, const RhsConst& P, int cj, int tag, double H[5],
-                                         double KK[5]) {
-  if (tag == 0) {
-    // Tam-Webb DRP, rhs_hybrid_high_llf.m4:258-268
-#pragma unroll
-    for (int k = 0; k < 5; ++k) {
-      // half fluxes in the planes: the coefficients are doubled (exactly)
-      double fx = 0.0, gy = 0.0;
-#pragma unroll
-      for (int m = 3; m >= 1; --m) {
-        const double a = 2.0 * (m == 1 ? Lit::a1 : (m == 2 ? Lit::a2 : Lit::a3));
-        fx = fma(a, A.fx(k, m) - A.fx(k, -m), fx);
-        gy = fma(a, A.gy(k, m) - A.gy(k, -m), gy);
-      }
-      KK[k] = (H[k] - fx * P.inv_dx0) - gy * P.inv_dx1;
+    for (int m = 3; m >= 1; --m) {
+      const double a = 2.0 * (m == 1 ? Lit::a1 : (m == 2 ? Lit::a2 : Lit::a3));
+      fx = fma(a, A.fx(k, m) - A.fx(k, -m), fx);
+      gy = fma(a, A.gy(k, m) - A.gy(k, -m), gy);
     }
+    D[k] = fma(fx, P.inv_dx0, gy * P.inv_dx1);
+  }
+}
+
+// Maximum of the magnitudes of n doubles of stride s around p (n odd), as
+// fmax gives it for numbers (magnitudes order as their bit patterns), on the
+// integer pipe.
+template <int QR>
+__device__ __forceinline__ double max_abs64(const double* p, int s) {
+  long long m = 0;
+#pragma unroll
+  for (int q = -QR; q <= QR; ++q) m = max(m, __double_as_longlong(p[q * s]) & 0x7fffffffffffffffll);
+  return __longlong_as_double(m);
+}
+
+// Half split speeds of a cell along x and y, rhs_hybrid_high_llf.m4:270-284.
+template <int ORDER, bool LLF, int TH>
+__device__ __forceinline__ void split_speeds64(const SAcc64P<TH>& A, const RhsConst& P, int cj, double& ha,
+                                               double& hb) {
+  if (!LLF) {
+    ha = hb = 0.5 * P.alpha;
     return;
   }
-  // split speeds, rhs_hybrid_high_llf.m4:270-284
-  double af, ag;
-  if (LLF) {
-    const int qr = ORDER == 5 ? 3 : 2;
-    double mx = 0.0;
-#pragma unroll
-    for (int q = -qr; q <= qr; ++q) mx = fmax(mx, fabs(A.u(q, 0)));
-    if (P.c_lr == 0.0) {
-      // (x + c) + 0 h is x + c, and x + c rounds monotonically in x: the
-      // maximum of the sums is the sum with the maximum (same doubles)
-      af = mx + P.c;
-      double mv = 0.0;
-#pragma unroll
-      for (int q = -qr; q <= qr; ++q) mv = fmax(mv, fabs(A.v(0, q)));
-      ag = mv + P.c;
-    } else {
-      const double hrow = P.ylo + P.dy * ((double)cj + 0.5);
-      af = (mx + P.c) + P.c_lr * hrow;
-      ag = 0.0;
-#pragma unroll
-      for (int q = -qr; q <= qr; ++q) {
-        const double h = P.ylo + P.dy * ((double)(cj + q) + 0.5);
-        ag = fmax(ag, (fabs(A.v(0, q)) + P.c) + P.c_lr * h);
-      }
-    }
+  constexpr int qr = ORDER == 5 ? 3 : 2;
+  const double mx = max_abs64<qr>(A.pl + A.c, 1);
+  if (P.c_lr == 0.0) {
+    // (x + c) + 0 h is x + c, and x + c rounds monotonically in x: the
+    // maximum of the sums is the sum with the maximum (same doubles)
+    ha = 0.5 * (mx + P.c);
+    hb = 0.5 * (max_abs64<qr>(A.pl + SAcc64P<TH>::G::OffV + A.c, kBW64) + P.c);
   } else {
-    af = P.alpha;
-    ag = P.alpha;
+    const double hrow = P.ylo + P.dy * ((double)cj + 0.5);
+    ha = 0.5 * ((mx + P.c) + P.c_lr * hrow);
+    double ag = 0.0;
+#pragma unroll
+    for (int q = -qr; q <= qr; ++q) {
+      const double h = P.ylo + P.dy * ((double)(cj + q) + 0.5);
+      ag = fmax(ag, (fabs(A.v(0, q)) + P.c) + P.c_lr * h);
+    }
+    hb = 0.5 * ag;
   }
-  const double ha = 0.5 * af, hb = 0.5 * ag;
-  KK[0] = weno_field64<ORDER>(A, P, 0, ha, hb, H[0]);
-  KK[1] = weno_field64<ORDER>(A, P, 1, ha, hb, H[1]);
-  KK[2] = weno_field64<ORDER>(A, P, 2, ha, hb, H[2]);
-  KK[3] = weno_field64<ORDER>(A, P, 3, ha, hb, H[3]);
-  KK[4] = weno_field64<ORDER>(A, P, 4, ha, hb, H[4]);
+}
+
+// The WENO cells of a tile, by the whole block of 256 threads: a task is one
+// field of up to 32 cells (one per lane), and the warps take the tasks in
+// turn, so a tile with few WENO cells still occupies every warp (a warp that
+// computed all five fields of its cells kept the other seven waiting at the
+// next barrier).  Tiles of one or two rows have fewer such tasks than warps:
+// there a task is one field along one direction.  `list` (cell indices cy * 32
+// + cx) holds the nw WENO cells of a mixed tile; without it every cell of the
+// w x h tile is one.  j0 is the index of the tile's first row for the height
+// of the split speeds.  D[p * 32 TH + cell] receives the flux part -(dF/dx +
+// dG/dy) of field p or, with one or two rows, -dF/dx of field p < 5 and -dG/dy
+// of field p - 5.
+template <int TH>
+constexpr int kFluxParts64 = TH <= 2 ? 10 : 5;
+template <int ORDER, bool LLF, int TH>
+__device__ __forceinline__ void weno_tasks64(const double* tile, const double* pl, const RhsConst& P, int j0, int w,
+                                             int h, const int* list, int nw, double* D) {
+  using G = Geo64<TH>;
+  constexpr int kParts = kFluxParts64<TH>;
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+  const int nchunk = list ? (nw + 31) >> 5 : h;
+  const double c = ORDER == 5 ? Lit::c1_6 : 0.5;
+  for (int t = warp; t < kParts * nchunk; t += 8) {
+    const int part = t / nchunk, q = t - part * nchunk;
+    int cell;
+    if (list) {
+      if (q * 32 + lane >= nw) continue;
+      cell = list[q * 32 + lane];
+    } else {
+      if (lane >= w) continue;
+      cell = q * 32 + lane;
+    }
+    const int cx = cell & 31, cy = cell >> 5;
+    const int k = kParts == 5 || part < 5 ? part : part - 5;
+    const SAcc64P<TH> A = acc64p<TH>(tile, pl, cx, cy);
+    double ha, hb;
+    split_speeds64<ORDER, LLF, TH>(A, P, j0 + cy, ha, hb);
+    const double* wk = tile + k * G::Pos + A.c;
+    const double* fk = pl + G::OffF + k * G::PF + A.cf;
+    const double* gk = pl + G::OffG + k * G::PG + A.cg;
+    double d;
+    if constexpr (kParts == 5) {
+      const double dfx = weno_flux64<ORDER>(wk, 1, fk, 1, ha);
+      const double dgy = weno_flux64<ORDER>(wk, kBW64, gk, 32, hb);
+      d = fma(dfx, P.inv_dx0, dgy * P.inv_dx1);
+    } else {
+      const bool y = part >= 5;
+      d = weno_flux64<ORDER>(wk, y ? kBW64 : 1, y ? gk : fk, y ? 32 : 1, y ? hb : ha) * (y ? P.inv_dx1 : P.inv_dx0);
+    }
+    D[part * (32 * TH) + cell] = c * d;
+  }
+}
+// dF/dx + dG/dy of field k of a WENO cell from weno_tasks64's parts.
+template <int TH>
+__device__ __forceinline__ double weno_part64(const double* D, int cell, int k) {
+  if constexpr (kFluxParts64<TH> == 5) return -D[k * (32 * TH) + cell];
+  else return -(D[k * (32 * TH) + cell] + D[(k + 5) * (32 * TH) + cell]);
 }
 
 // Accessor of the learned switch's features on an FP64 tile: density and
@@ -351,10 +339,11 @@ struct SAcc64Feat {
   const double* t;
   int c;
   double rho0, p0;
+  static constexpr int kPos = Geo64<8>::Pos;
   __device__ float w(int k, int di, int dj) const {
-    return (float)(t[k * kPos64 + c + dj * kBW64 + di] - (k == 0 ? rho0 : 0.0));
+    return (float)(t[k * kPos + c + dj * kBW64 + di] - (k == 0 ? rho0 : 0.0));
   }
-  __device__ float p(int di, int dj) const { return (float)(t[5 * kPos64 + c + dj * kBW64 + di] - p0); }
+  __device__ float p(int di, int dj) const { return (float)(t[5 * kPos + c + dj * kBW64 + di] - p0); }
 };
 
 }  // namespace enl

@@ -88,11 +88,15 @@ constexpr int kOffTile32 = 2 * kStageBufBytes;
 constexpr int kOffPlanes = kOffTile32 + kTile32Bytes;
 constexpr int kSmemFast64 = kOffPlanes + kPlanesBytes;   // dynamic shared memory, FP64 storage + FP32 rhs
 constexpr int kOffPlanesS = 2 * kBufS;
-// FP64 right-hand side: [FP64 box A][FP64 box B][FP64 planes]
+// FP64 right-hand side: [FP64 box A][FP64 box B][FP64 planes][flux parts]:
+// the planes of u, v and the half fluxes,
+// and the WENO cells' flux parts (5 fields of the tile's cells)
+using Geo = Geo64<kTH>;
 constexpr int kOffPlanes64 = 2 * kStageBufBytes;
-constexpr int kPlanes64Bytes = align128(kPl64Elems * 8);               // 38656
-constexpr int kSmem64 = kOffPlanes64 + kPlanes64Bytes;                  // dynamic shared memory, FP64
-static_assert(kBH * kBW == kPos64 && kBW == kBW64, "FP64 planes follow the staged box");
+constexpr int kPlanes64Bytes = align128(Geo::Elems * 8);               // 38656
+constexpr int kOffFlux64 = kOffPlanes64 + kPlanes64Bytes;
+constexpr int kSmem64 = kOffFlux64 + 5 * kTH * kTW * 8;                 // dynamic shared memory, FP64
+static_assert(kBH * kBW == Geo::Pos && kBW == kBW64, "FP64 planes follow the staged box");
 constexpr int kSmemFast32 = kOffPlanesS + kPlanesBytes;  // dynamic shared memory, FP32 storage
 constexpr unsigned long long kWaitNs = 200000000ull;  // bounded mbarrier waits: 0.2 s of wall time
 // learned switch: cells per network chunk (8 warps x 16 cells); their BF16
@@ -100,7 +104,7 @@ constexpr unsigned long long kWaitNs = 200000000ull;  // bounded mbarrier waits:
 // again after it
 constexpr int kFeatRows = 128;
 static_assert(kFeatRows * kFeat * 2 <= kPlanesBytes, "the features fit where the planes go");
-static_assert(kFeatRows * kFeat * 2 <= align128(kPl64Elems * 8), "the features fit where the FP64 planes go");
+static_assert(kFeatRows * kFeat * 2 <= kPlanes64Bytes, "the features fit where the FP64 planes go");
 // Resident stage blocks per SM with FP32 storage (bounds the registers per
 // thread: 4 blocks of 256 threads leave 64, 3 leave 80).  Four blocks need
 // the smaller staging buffers of ENL_STAGE_UN_TMA 0 (4 x 56 KB of shared
@@ -672,6 +676,7 @@ __global__ void __launch_bounds__(256, std::is_same<S, float>::value ? kStageBlo
   float* tile32_conv = reinterpret_cast<float*>(smem_raw + kOffTile32);  // FP64 storage, FAST
   float* planes = reinterpret_cast<float*>(smem_raw + (kF32S ? kOffPlanesS : kOffPlanes));  // FAST
   double* planes64 = reinterpret_cast<double*>(smem_raw + kOffPlanes64);  // FP64 right-hand side
+  double* flux64 = reinterpret_cast<double*>(smem_raw + kOffFlux64);
   // learned sensor (hybrid only): features of up to kFeatRows cells at a
   // time in the planes' place; the network image stays in global memory
   __nv_bfloat16* feat = reinterpret_cast<__nv_bfloat16*>(FAST ? (void*)planes : (void*)planes64);
@@ -876,7 +881,7 @@ __global__ void __launch_bounds__(256, std::is_same<S, float>::value ? kStageBlo
           SAcc32R acc{acc32(tile32, planes, tx, ty)};
           flag = SCHEME == kWeno ? 1 : (SCHEME == kDrp ? 0 : sensor_fast(acc, A.F[lvl]));
         } else {
-          flag = switch64<SCHEME>(acc64p(tile, planes64, tx, ty), A.P[lvl]);
+          flag = switch64<SCHEME, kTH>(acc64p<kTH>(tile, planes64, tx, ty), A.P[lvl]);
         }
       }
       unsigned bd = __ballot_sync(0xffffffffu, valid && !flag);
@@ -909,31 +914,7 @@ __global__ void __launch_bounds__(256, std::is_same<S, float>::value ? kStageBlo
             }
           }
         } else {
-          // FP64: one seeded reciprocal of rho per halo position; the flux
-          // planes hold half fluxes, formed from u/2, v/2 and p/2 (halving
-          // is exact, so each is F/2 or G/2 of the same double)
-          for (int e = 255 - tid; e < kPos64; e += 256) {
-            const int row = e / kBW64, col = e - row * kBW64;
-            const double ir = rcp64(tile[e]);
-            const double u = tile[kPos64 + e] * ir, v = tile[2 * kPos64 + e] * ir;
-            const double hp = 0.5 * tile[5 * kPos64 + e];
-            planes64[e] = u;
-            planes64[kPl64OffV + e] = v;
-            if (row >= 3 && row < 3 + kTH) {
-              const double hu = 0.5 * u;
-#pragma unroll
-              for (int k = 0; k < 5; ++k)
-                planes64[kPl64OffF + k * kPl64F + (row - 3) * kBW64 + col] =
-                    k == 1 ? fma(hu, tile[kPos64 + e], hp) : hu * tile[k * kPos64 + e];
-            }
-            if (col >= 3 && col < 3 + kTW) {
-              const double hv = 0.5 * v;
-#pragma unroll
-              for (int k = 0; k < 5; ++k)
-                planes64[kPl64OffG + k * kPl64G + row * kTW + (col - 3)] =
-                    k == 2 ? fma(hv, tile[2 * kPos64 + e], hp) : hv * tile[k * kPos64 + e];
-            }
-          }
+          build_planes64<kTH>(tile, planes64, w, h);
         }
       };
       // the learned review (tiles with WENO cells on level 0, or on every
@@ -1032,21 +1013,36 @@ __global__ void __launch_bounds__(256, std::is_same<S, float>::value ? kStageBlo
         build_planes();  // the features took the planes' place
         __syncthreads();
       }
-      // a tile without WENO cells keeps its natural order (no list, no barrier)
-      const bool direct = SCHEME == kWeno || nw == 0;  // one branch for the whole tile
-      if (valid && !direct) {
-        unsigned lt = (1u << lane) - 1u;
-        int pos = flag ? (nd + ow + __popc(bw & lt)) : (od + __popc(bd & lt));
-        s_list[pos] = (ty << 5) | tx | (flag << 16);
-      }
       if (tid == 0) {  // per-block counts, added to A.stats when the block leaves
         s_stats[4 * lvl + 0] += (unsigned)nw;
         s_stats[4 * lvl + 1] += (unsigned)(nd + nw);
         s_stats[4 * lvl + 2] += (unsigned)nfb;
       }
-      if (!direct) __syncthreads();
+      // FP32 right-hand side: the cells are reordered so that every warp runs
+      // one branch, and a thread finishes the cell it is given.  FP64: the
+      // block computes the WENO cells' flux parts field by field, then every
+      // thread finishes its own cell (stores stay coalesced).  A tile without
+      // WENO cells (and one of a WENO-only scheme) keeps its natural order: no
+      // list, no barrier.
+      const bool direct = !FAST || SCHEME == kWeno || nw == 0;
+      if constexpr (FAST) {
+        if (valid && !direct) {
+          unsigned lt = (1u << lane) - 1u;
+          int pos = flag ? (nd + ow + __popc(bw & lt)) : (od + __popc(bd & lt));
+          s_list[pos] = (ty << 5) | tx | (flag << 16);
+        }
+        if (!direct) __syncthreads();
+      } else if (nw > 0) {
+        const bool all = SCHEME == kWeno || nw == w * h;
+        if (!all) {
+          if (valid && flag) s_list[ow + __popc(bw & ((1u << lane) - 1u))] = (ty << 5) | tx;
+          __syncthreads();
+        }
+        weno_tasks64<ORDER, LLF, kTH>(tile, planes64, A.P[lvl], j0, w, h, all ? nullptr : s_list, nw, flux64);
+        __syncthreads();
+      }
       if (direct ? valid : (tid < nd + nw)) {
-        const int e = direct ? ((ty << 5) | tx | (SCHEME == kWeno ? 1 << 16 : 0)) : s_list[tid];
+        const int e = direct ? ((ty << 5) | tx | (FAST ? (SCHEME == kWeno ? 1 << 16 : 0) : flag << 16)) : s_list[tid];
         const int cx = e & 31, cy = (e >> 5) & 0xff, f = (e >> 16) & 1;
         const int c2 = (cy + 3) * kBW + (cx + 3);
         const int c32 = (cy + 3) * kBW32 + (cx + 3);
@@ -1130,15 +1126,20 @@ __global__ void __launch_bounds__(256, std::is_same<S, float>::value ? kStageBlo
             pv = A.p0 + (double)pp;
             tv = A.T0 + (double)tp;
           } else {
-            SAcc64P acc = acc64p(tile, planes64, cx, cy);
-            double H[5], K[5];
+            const SAcc64P<kTH> acc = acc64p<kTH>(tile, planes64, cx, cy);
+            double H[5], D[5];
             H[0] = static_cast<const double*>(A.h0[lvl])[g];
             sources64(acc, A.P[lvl], H);
-            fluxes64<ORDER, LLF>(acc, A.P[lvl], gj, f, H, K);
+            if (f) {
+#pragma unroll
+              for (int k = 0; k < 5; ++k) D[k] = weno_part64<kTH>(flux64, tid, k);
+            } else {
+              drp_flux64(acc, A.P[lvl], D);
+            }
 #pragma unroll
             for (int k = 0; k < 5; ++k) {
               double win = tile[k * (kBH * kBW) + c2];
-              wn[k] = (A.a1 * un[k * fs + g] + A.a2 * win) + bdt * K[k];
+              wn[k] = (A.a1 * un[k * fs + g] + A.a2 * win) + bdt * (H[k] - D[k]);
             }
             // update_state (update_state.m4:90-105), as the state upload computes it
             eos_fast64(A.E64, wn[0], wn[3], row_height64(A.ylo, A.dy[lvl], gj), pv, tv);
