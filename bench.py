@@ -755,7 +755,7 @@ def run_ours(args):
         "config": {"workload": wl.name, "path": "plain FP64, drop-in F77 ABI", "cells": wl.cells,
                    "l2": "flushed between timed steps (512 MB write)", "parallelism": "replicas" if ws > 1 else "1 GPU"},
         "roofline": {"bound": "hbm", "achieved": achieved, "peak": hbm_peak, "unit": "GB/s",
-                     "frac": achieved / hbm_peak, "traffic": traffic, "kernel": "rhs_plain_kernel",
+                     "frac": achieved / hbm_peak, "traffic": traffic, "kernel": "rhs_tile_kernel",
                      "peak_kind": peak_kind, "bytes_per_cell": RHS_BYTES_PER_CELL, "kernel_ms": rhs_ms},
         "step_roofline": {"bytes_per_cell_update": STEP_BYTES_PER_CELL,
                           "frac": value * STEP_BYTES_PER_CELL / (hbm_peak * 1e9)},

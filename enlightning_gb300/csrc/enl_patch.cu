@@ -1,6 +1,6 @@
 // Per-patch FP64 kernels behind the drop-in F77 entry points.
 //
-//   rhs_           fortran/rhs_*.m4           (rhs_plain_kernel)
+//   rhs_           fortran/rhs_*.m4           (rhs_tile_kernel)
 //   runge_kutta_   fortran/runge_kutta.m4     (runge_kutta_kernel)
 //   update_state_  fortran/update_state.m4    (update_state_kernel)
 //   tag_cells_     fortran/tag_cells.m4       (tag_cells_kernel)
@@ -13,43 +13,91 @@
 #include <cmath>
 #include <cstdio>
 
-#include "enl_rhs_cell.cuh"
+#include "enl_cell64.cuh"
 
 namespace enl {
 
 int rhs_variant();
 
-// Global-memory accessor centred on one cell.
-struct GAcc {
-  const double* wp;  // field 0 at the centre cell
-  const double* pr;  // pressure at the centre cell
-  const double* te;  // temperature at the centre cell
-  long pitch, fstride;
-  __device__ double w(int k, int di, int dj) const { return __ldg(wp + k * fstride + dj * pitch + di); }
-  __device__ double p(int di, int dj) const { return __ldg(pr + dj * pitch + di); }
-  __device__ double t(int di, int dj) const { return __ldg(te + dj * pitch + di); }
-};
-
-template <int SCHEME, int ORDER, bool LLF>
-__global__ void __launch_bounds__(128) rhs_plain_kernel(const double* __restrict__ w, const double* __restrict__ pres,
-                                         const double* __restrict__ temp, long pitch, long fstride, int g0,
-                                         int g1, const double* __restrict__ H0, double* __restrict__ KK,
-                                         long opitch, long ofstride, int nx, int ny, RhsConst P,
-                                         int* __restrict__ flags) {
-  int ci = blockIdx.x * blockDim.x + threadIdx.x;
-  int cj = blockIdx.y * blockDim.y + threadIdx.y;
-  if (ci >= nx || cj >= ny) return;
-  long c = (long)(cj + g1) * pitch + (ci + g0);
-  GAcc A{w + c, pres + c, temp + c, pitch, fstride};
-  int tag = rhs_switch<SCHEME, ORDER, LLF>(A, P);
-  double H[5], K[5];
-  H[0] = H0[(long)cj * opitch + ci];
-  rhs_sources(A, P, H);
-  rhs_fluxes<SCHEME, ORDER, LLF>(A, P, cj, tag, H, K);
-  long o = (long)cj * opitch + ci;
+// The right-hand side of one patch, by tiles of 32 x TH cells, one block of
+// 256 threads each: the block copies the halo box of the 7 fields into shared
+// memory (8-byte asynchronous copies: a patch's rows start anywhere, so
+// neither wider copies nor TMA boxes fit them), forms velocities and half
+// fluxes once per position, computes the flux parts of its WENO cells field by
+// field (weno_tasks64), and every thread finishes one cell.  The arithmetic is
+// the batched engine's (enl_cell64.cuh).  Bound by the FP64 and FP32 pipes.
+// One thread per cell reading the patch through L1, with 23 FP64 divisions and
+// 40 FP64 reconstructions a WENO cell, took 430 us on 512x512 (hybrid, level
+// 0), 129 us on 131x93 (fine level) and 111 us on 24x16; this takes 171, 35
+// and 25 us.
+//
+// TH: 8 rows for large patches (the least work for the halo: 14 rows of
+// planes for 8 of cells); fewer rows when the patch has too few tiles for the
+// SMs (rhs_rows).
+template <int SCHEME, int ORDER, bool LLF, int TH>
+__global__ void __launch_bounds__(256, 2)
+    rhs_tile_kernel(const double* __restrict__ w, const double* __restrict__ pres, const double* __restrict__ temp,
+                    long pitch, long fstride, int g0, int g1, const double* __restrict__ H0, double* __restrict__ KK,
+                    long opitch, long ofstride, int nx, int ny, const __grid_constant__ RhsConst P,
+                    int* __restrict__ flags) {
+  using G = Geo64<TH>;
+  extern __shared__ __align__(16) double sm[];
+  double* tile = sm;
+  double* pl = tile + 7 * G::Pos;
+  double* flux = pl + G::Elems;
+  __shared__ int s_list[32 * TH];
+  __shared__ int s_cnt[8];
+  const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+  const int i0 = blockIdx.x * 32, j0 = blockIdx.y * TH;
+  const int tw = min(32, nx - i0), th = min(TH, ny - j0);
+  const long o0 = (long)(j0 + g1 - 3) * pitch + (i0 + g0 - 3);
+  for (int e = tid; e < 7 * G::Pos; e += 256) {
+    const int k = e / G::Pos, r = e - k * G::Pos, row = r / kBW64, col = r - row * kBW64;
+    if (row < th + 6 && col < tw + 6) {
+      const double* src = (k < 5 ? w + k * fstride : (k == 5 ? pres : temp)) + o0 + row * pitch + col;
+      asm volatile("cp.async.ca.shared.global [%0], [%1], 8;" ::"r"((unsigned)__cvta_generic_to_shared(tile + e)),
+                   "l"(src));
+    }
+  }
+  asm volatile("cp.async.wait_all;" ::: "memory");
+  __syncthreads();
+  const bool valid = warp < th && lane < tw;
+  int flag = 0;
+  if (valid) flag = switch64<SCHEME, TH>(acc64p<TH>(tile, pl, lane, warp), P);
+  build_planes64<TH>(tile, pl, tw, th);
+  const unsigned bw = __ballot_sync(0xffffffffu, valid && flag);
+  if (lane == 0) s_cnt[warp] = __popc(bw);
+  __syncthreads();
+  int nw = 0, ow = 0;
 #pragma unroll
-  for (int k = 0; k < 5; ++k) KK[k * ofstride + o] = K[k];
-  if (flags) flags[o] = tag;
+  for (int q = 0; q < (TH < 8 ? TH : 8); ++q) {
+    if (q < warp) ow += s_cnt[q];
+    nw += s_cnt[q];
+  }
+  if (SCHEME != kDrp && nw > 0) {
+    const bool all = nw == tw * th;
+    if (!all) {
+      if (valid && flag) s_list[ow + __popc(bw & ((1u << lane) - 1u))] = tid;
+      __syncthreads();
+    }
+    weno_tasks64<ORDER, LLF, TH>(tile, pl, P, j0, tw, th, all ? nullptr : s_list, nw, flux);
+    __syncthreads();
+  }
+  if (!valid) return;
+  const SAcc64P<TH> A = acc64p<TH>(tile, pl, lane, warp);
+  const long o = (long)(j0 + warp) * opitch + (i0 + lane);
+  double H[5], D[5];
+  H[0] = H0[o];
+  sources64(A, P, H);
+  if (flag) {
+#pragma unroll
+    for (int k = 0; k < 5; ++k) D[k] = weno_part64<TH>(flux, tid, k);
+  } else {
+    drp_flux64(A, P, D);
+  }
+#pragma unroll
+  for (int k = 0; k < 5; ++k) KK[k * ofstride + o] = H[k] - D[k];
+  if (flags) flags[o] = flag;
 }
 
 // runge_kutta.m4:60-63, association kept: (a1*ww + a2*w_n) + (beta*dt)*KK.
@@ -267,30 +315,73 @@ RhsConst make_rhs_const(const double* xlo, const double* dx, double alpha, doubl
   return P;
 }
 
-static int launch_rhs(int variant, dim3 grid, dim3 block, const double* w, const double* pres,
-                      const double* temp, long pitch, long fstride, int g0, int g1, const double* H0,
-                      double* KK, long opitch, long ofstride, int nx, int ny, const RhsConst& P, int* flags) {
-  cudaStream_t s = stream();
-#define ENL_RHS_CASE(ID, SCH, ORD, LLF_)                                                              \
-  case ID:                                                                                           \
-    rhs_plain_kernel<SCH, ORD, LLF_><<<grid, block, 0, s>>>(w, pres, temp, pitch, fstride, g0, g1, H0, \
-                                                            KK, opitch, ofstride, nx, ny, P, flags); \
-    break;
+// Rows per tile.  With fewer rows more blocks share a patch, and each does more
+// work for its halo (TH + 6 rows of planes for TH of cells).  Two blocks run on
+// an SM.  Measured, hybrid scheme on level 0 / on a fine level (WENO in every
+// cell), us for 8, 4, 2, 1 rows:
+//   32x32    73 43 29 25    / 66 38 25 19
+//   131x93   76 44 42 52    / 66 39 35 48
+//   256x256  87 76 74 113   / 105 109 111 146
+//   384x384  130 108 127 213 / 202 206 236 312
+//   512x512  179 171 205 351 / 336 334 390 534
+//   700x700  280 299 356 617 / 588 592 704 983
+// so 8 rows from four waves of blocks on, 4 from one wave, 2 from half a wave.
+static int rhs_rows(int nx, int ny) {
+  const long cols = (nx + 31) / 32;
+  int dev = 0, nsm = 1;
+  cudaGetDevice(&dev);
+  cudaDeviceGetAttribute(&nsm, cudaDevAttrMultiProcessorCount, dev);
+  if (cols * ((ny + 7) / 8) >= 8l * nsm) return 8;
+  if (cols * ((ny + 3) / 4) >= 2l * nsm) return 4;
+  return cols * ((ny + 1) / 2) >= nsm ? 2 : 1;
+}
+
+struct RhsCall {
+  const double *w, *pres, *temp;
+  long pitch, fstride;
+  int g0, g1;
+  const double* H0;
+  double* KK;
+  long opitch, ofstride;
+  int nx, ny;
+  int* flags;
+};
+
+template <int SCHEME, int ORDER, bool LLF, int TH>
+static void launch_rhs_rows(const RhsCall& c, const RhsConst& P) {
+  constexpr size_t bytes = (7 * Geo64<TH>::Pos + Geo64<TH>::Elems + kFluxParts64<TH> * 32 * TH) * sizeof(double);
+  auto fn = rhs_tile_kernel<SCHEME, ORDER, LLF, TH>;
+  if (bytes > 48 * 1024) cudaFuncSetAttribute((const void*)fn, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)bytes);
+  const dim3 grid((c.nx + 31) / 32, (c.ny + TH - 1) / TH);
+  fn<<<grid, 256, bytes, stream()>>>(c.w, c.pres, c.temp, c.pitch, c.fstride, c.g0, c.g1, c.H0, c.KK, c.opitch,
+                                     c.ofstride, c.nx, c.ny, P, c.flags);
+}
+
+template <int SCHEME, int ORDER, bool LLF>
+static void launch_rhs_scheme(const RhsCall& c, const RhsConst& P) {
+  switch (rhs_rows(c.nx, c.ny)) {
+    case 8: return launch_rhs_rows<SCHEME, ORDER, LLF, 8>(c, P);
+    case 4: return launch_rhs_rows<SCHEME, ORDER, LLF, 4>(c, P);
+    case 2: return launch_rhs_rows<SCHEME, ORDER, LLF, 2>(c, P);
+    default: return launch_rhs_rows<SCHEME, ORDER, LLF, 1>(c, P);
+  }
+}
+
+static int launch_rhs(int variant, const RhsCall& c, const RhsConst& P) {
   switch (variant) {
-    ENL_RHS_CASE(0, kHybrid, 5, true)
-    ENL_RHS_CASE(1, kHybrid, 5, false)
-    ENL_RHS_CASE(2, kHybrid, 3, true)
-    ENL_RHS_CASE(3, kHybrid, 3, false)
-    ENL_RHS_CASE(4, kWeno, 5, true)
-    ENL_RHS_CASE(5, kWeno, 5, false)
-    ENL_RHS_CASE(6, kWeno, 3, true)
-    ENL_RHS_CASE(7, kWeno, 3, false)
-    ENL_RHS_CASE(8, kDrp, 5, false)
+    case 0: launch_rhs_scheme<kHybrid, 5, true>(c, P); break;
+    case 1: launch_rhs_scheme<kHybrid, 5, false>(c, P); break;
+    case 2: launch_rhs_scheme<kHybrid, 3, true>(c, P); break;
+    case 3: launch_rhs_scheme<kHybrid, 3, false>(c, P); break;
+    case 4: launch_rhs_scheme<kWeno, 5, true>(c, P); break;
+    case 5: launch_rhs_scheme<kWeno, 5, false>(c, P); break;
+    case 6: launch_rhs_scheme<kWeno, 3, true>(c, P); break;
+    case 7: launch_rhs_scheme<kWeno, 3, false>(c, P); break;
+    case 8: launch_rhs_scheme<kDrp, 5, false>(c, P); break;
     default:
       set_error(ENL_ERR_ARG);
       return ENL_ERR_ARG;
   }
-#undef ENL_RHS_CASE
   return check_launch("rhs");
 }
 
@@ -299,10 +390,8 @@ static int launch_rhs(int variant, dim3 grid, dim3 block, const double* w, const
 int launch_rhs_pitched(int variant, const double* w, const double* pres, const double* temp, long pitch,
                        long fstride, const double* H0, double* KK, long opitch, long ofstride, int nx, int ny,
                        const RhsConst& P) {
-  dim3 block(32, 4);
-  dim3 grid((nx + block.x - 1) / block.x, (ny + block.y - 1) / block.y);
-  return launch_rhs(variant, grid, block, w, pres, temp, pitch, fstride, 3, 3, H0, KK, opitch, ofstride, nx, ny, P,
-                    nullptr);
+  return launch_rhs(variant, RhsCall{w, pres, temp, pitch, fstride, 3, 3, H0, KK, opitch, ofstride, nx, ny, nullptr},
+                    P);
 }
 
 }  // namespace enl
@@ -327,9 +416,9 @@ int enl_rhs(int variant, int ifirst0, int ilast0, int ifirst1, int ilast1, int g
   }
   RhsConst P = make_rhs_const(xlo, dx, weno_alpha, kappa, mu, muB, R, T_star_n, tau_n, tag_tolerance, level,
                               c, c_lr);
-  dim3 block(32, 4);
-  return launch_rhs(variant, grid2d(nx, ny, block), block, w_n, pressure, temperature, w_pitch, w_fstride,
-                    gcw0, gcw1, source, rhs, out_pitch, out_fstride, nx, ny, P, flags);
+  return launch_rhs(variant, RhsCall{w_n, pressure, temperature, w_pitch, w_fstride, gcw0, gcw1, source, rhs,
+                                     out_pitch, out_fstride, nx, ny, flags},
+                    P);
 }
 
 void rhs_(const int& ifirst0, const int& ilast0, const int& ifirst1, const int& ilast1, const int& gcw0,
