@@ -4,12 +4,14 @@
 //   runge_kutta_   fortran/runge_kutta.m4     (runge_kutta_kernel)
 //   update_state_  fortran/update_state.m4    (update_state_kernel)
 //   tag_cells_     fortran/tag_cells.m4       (tag_cells_kernel)
-//   enl_phys_bc    enlightning.C:790-1013     (phys_bc_edge_kernel, phys_bc_node_kernel)
-//   enl_absorb     enlightning.C:634-786      (absorb_x_kernel, absorb_y_kernel)
+//   enl_phys_bc    enlightning.C:790-1013     (phys_bc_kernel)
+//   enl_absorb     enlightning.C:634-786      (absorb_kernel)
 //
 // Every kernel addresses its patch through a pitched view (first stored cell,
 // row pitch, field stride) so that the same code serves SAMRAI's contiguous
 // CellData arrays and patches embedded in a larger level array.
+#include <algorithm>
+#include <climits>
 #include <cmath>
 #include <cstdio>
 
@@ -101,19 +103,32 @@ __global__ void __launch_bounds__(256, 2)
 }
 
 // runge_kutta.m4:60-63, association kept: (a1*ww + a2*w_n) + (beta*dt)*KK.
-__global__ void runge_kutta_kernel(double* __restrict__ wn, long pitch, long fstride, int g0, int g1,
-                                   const double* __restrict__ ww, const double* __restrict__ KK,
-                                   long ipitch, long ifstride, int nx, int ny, int nequ, double a1,
-                                   double a2, double bdt) {
-  int ci = blockIdx.x * blockDim.x + threadIdx.x;
-  int cj = blockIdx.y * blockDim.y + threadIdx.y;
-  if (ci >= nx || cj >= ny) return;
-  long g = (long)(cj + g1) * pitch + (ci + g0);
-  long c = (long)cj * ipitch + ci;
-  for (int k = 0; k < nequ; ++k) {
-    double v = __dadd_rn(__dadd_rn(__dmul_rn(a1, ww[k * ifstride + c]), __dmul_rn(a2, wn[k * fstride + g])),
-                         __dmul_rn(bdt, KK[k * ifstride + c]));
-    wn[k * fstride + g] = v;
+// Bound by memory: blockIdx.z takes one field, and a thread has the loads of
+// kRkCells cells (32 columns apart) in flight at once.
+constexpr int kRkCells = 4;
+__global__ void __launch_bounds__(128) runge_kutta_kernel(double* __restrict__ wn, long pitch, long fstride, int g0,
+                                                          int g1, const double* __restrict__ ww,
+                                                          const double* __restrict__ KK, long ipitch, long ifstride,
+                                                          int nx, int ny, double a1, double a2, double bdt) {
+  const int ci = blockIdx.x * (32 * kRkCells) + threadIdx.x, cj = blockIdx.y * blockDim.y + threadIdx.y;
+  if (cj >= ny) return;
+  double* wr = wn + blockIdx.z * fstride + (long)(cj + g1) * pitch + g0;
+  const double* ur = ww + blockIdx.z * ifstride + (long)cj * ipitch;
+  const double* kr = KK + blockIdx.z * ifstride + (long)cj * ipitch;
+  double u[kRkCells], w[kRkCells], k[kRkCells];
+#pragma unroll
+  for (int q = 0; q < kRkCells; ++q) {
+    const int i = ci + 32 * q;
+    if (i < nx) {
+      u[q] = ur[i];
+      w[q] = wr[i];
+      k[q] = kr[i];
+    }
+  }
+#pragma unroll
+  for (int q = 0; q < kRkCells; ++q) {
+    const int i = ci + 32 * q;
+    if (i < nx) wr[i] = __dadd_rn(__dadd_rn(__dmul_rn(a1, u[q]), __dmul_rn(a2, w[q])), __dmul_rn(bdt, k[q]));
   }
 }
 
@@ -167,61 +182,95 @@ __global__ void tag_cells_kernel(int* __restrict__ tags, long tpitch, const doub
   tags[(long)cj * tpitch + ci] = t ? tag_val : 0;
 }
 
-// Physical-boundary fill, enlightning.C:830-944 (edges).  Each ghost cell of
-// an edge box receives the first interior cell of its row/column (the
-// reference's cascading copy), the normal momentum negated on REFLECT sides.
-// One thread per (tangential cell, ghost depth, field).  The fields array
-// holds w_n (5), pressure, temperature, source: 8 pointers.
+// Physical-boundary fill, enlightning.C:830-1008.  Each ghost cell of an edge
+// box receives the first interior cell of its row or column (the reference's
+// cascading copy), the normal momentum negated on REFLECT sides.  The nodes
+// (corners) then copy along x from the cell next to the corner box, an edge
+// ghost or a neighbour-filled one, x-momentum negated when the adjacent x side
+// is REFLECT.  An edge ghost is itself a copy of an interior cell, so a node
+// takes that cell's value and no ghost is read that this kernel writes: edges
+// and nodes go in one launch (they were up to eight: 3 us each on the GPU and
+// as much on the host for a 24x16 patch's 12 us of arithmetic).  The fields
+// are w_n (5), pressure, temperature, source; blockIdx.y picks one.
 struct PatchFields8 {
   double* f[8];
 };
 
-__global__ void phys_bc_edge_kernel(PatchFields8 F, long pitch, int nx, int ny, int g0, int g1, int side,
-                                    int fill, int reflect) {
-  int t = blockIdx.x * blockDim.x + threadIdx.x;
-  int tan_n = (side < 2) ? ny : nx;
-  int total = tan_n * fill * 8;
-  if (t >= total) return;
-  int k = t % 8;
-  int d = (t / 8) % fill;       // depth 0 = adjacent ghost
-  int s = t / (8 * fill);       // tangential index
-  int i, j, si, sj;
-  if (side == 0) { j = s + g1; i = g0 - 1 - d; si = g0; sj = j; }
-  else if (side == 1) { j = s + g1; i = g0 + nx + d; si = g0 + nx - 1; sj = j; }
-  else if (side == 2) { i = s + g0; j = g1 - 1 - d; si = i; sj = g1; }
-  else { i = s + g0; j = g1 + ny + d; si = i; sj = g1 + ny - 1; }
-  double v = F.f[k][(long)sj * pitch + si];
-  int neg_k = (side < 2) ? 1 : 2;
-  if (k == neg_k && reflect) v = -v;
-  F.f[k][(long)j * pitch + i] = v;
-}
+struct BandArgs {
+  PatchFields8 F;
+  long pitch;
+  int nx, ny, g0, g1, fill0, fill1;
+  int touches, reflect;  // bit per side L, R, B, T
+  int cells;             // band cells of the sides touched and of their nodes
+};
 
-// Nodes (corners), enlightning.C:948-1008: copy along x from the cell next
-// to the corner box (an edge ghost or a neighbour-filled ghost), x-momentum
-// negated when the adjacent x side is REFLECT.
-__global__ void phys_bc_node_kernel(PatchFields8 F, long pitch, int nx, int ny, int g0, int g1, int loc,
-                                    int fill0, int fill1, int reflect_x) {
-  int t = blockIdx.x * blockDim.x + threadIdx.x;
-  int total = fill0 * fill1 * 8;
-  if (t >= total) return;
-  int k = t % 8;
-  int dx = (t / 8) % fill0;
-  int dy = t / (8 * fill0);
-  int xs = loc & 1, ys = (loc >> 1) & 1;
-  int j = ys ? (g1 + ny + dy) : (g1 - 1 - dy);
-  int i = xs ? (g0 + nx + dx) : (g0 - 1 - dx);
-  int si = xs ? (g0 + nx - 1) : g0;
-  double v = F.f[k][(long)j * pitch + si];
-  if (k == 1 && reflect_x) v = -v;
-  F.f[k][(long)j * pitch + i] = v;
+__global__ void phys_bc_kernel(const __grid_constant__ BandArgs A) {
+  const int k = blockIdx.y;
+  double* f = A.F.f[k];
+  for (int t = blockIdx.x * blockDim.x + threadIdx.x; t < A.cells; t += gridDim.x * blockDim.x) {
+    int r = t, i = -1, j = -1, si = 0, sj = 0;
+    bool neg = false;
+    const int nsx = A.ny * A.fill0, nsy = A.nx * A.fill1, nn = A.fill0 * A.fill1;
+#pragma unroll
+    for (int side = 0; side < 4; ++side) {
+      if (!(A.touches & (1 << side)) || i >= 0) continue;
+      const int n = side < 2 ? nsx : nsy;
+      if (r >= n) {
+        r -= n;
+        continue;
+      }
+      if (side < 2) {
+        const int d = r % A.fill0;
+        sj = j = r / A.fill0 + A.g1;
+        si = side == 0 ? A.g0 : A.g0 + A.nx - 1;
+        i = side == 0 ? A.g0 - 1 - d : A.g0 + A.nx + d;
+        neg = k == 1 && (A.reflect & (1 << side));
+      } else {
+        const int d = r / A.nx;
+        si = i = r - d * A.nx + A.g0;
+        sj = side == 2 ? A.g1 : A.g1 + A.ny - 1;
+        j = side == 2 ? A.g1 - 1 - d : A.g1 + A.ny + d;
+        neg = k == 2 && (A.reflect & (1 << side));
+      }
+    }
+    if (i < 0) {
+#pragma unroll
+      for (int loc = 0; loc < 4; ++loc) {
+        const int xs = loc & 1, ys = 2 + (loc >> 1);
+        if (!((A.touches >> xs | A.touches >> ys) & 1) || i >= 0) continue;
+        if (r >= nn) {
+          r -= nn;
+          continue;
+        }
+        const int dx = r % A.fill0, dy = r / A.fill0;
+        j = ys == 3 ? A.g1 + A.ny + dy : A.g1 - 1 - dy;
+        i = xs ? A.g0 + A.nx + dx : A.g0 - 1 - dx;
+        si = xs ? A.g0 + A.nx - 1 : A.g0;
+        // the row's ghost beside the node: filled from the interior when the
+        // patch touches that side, a neighbour's cell otherwise
+        const bool filled = (A.touches >> ys) & 1;
+        sj = filled ? (ys == 3 ? A.g1 + A.ny - 1 : A.g1) : j;
+        neg = (k == 1 && ((A.reflect >> xs) & 1)) != (k == 2 && filled && ((A.reflect >> ys) & 1));
+      }
+    }
+    const double v = f[(long)sj * A.pitch + si];
+    f[(long)j * A.pitch + i] = neg ? -v : v;
+  }
 }
 
 // Absorbing envelope, enlightning.C:671-783, including the loop-exit rules:
 // along x each row runs from the boundary side while the previous envelope
 // value differs from 1 by more than 1e-8 (the first row starts from the
 // envelope of the first cell, later rows from tmp = 0); along y the same rule
-// runs over rows.  dir: 0 = L, 1 = R (one thread per row); 2 = B, 3 = T (one
-// thread per column, each walking the rows).
+// runs over rows.  dir: 0 = L, 1 = R, 2 = B, 3 = T.
+//
+// The distance from the side grows along the walk, and the envelope with it,
+// so whether the walk reaches a cell follows from the cell before it alone:
+// one thread per cell applies the sides that reach it in the reference's
+// order.  A block covers 32 x 8 cells and computes the factors of its columns
+// and rows once; blocks that no side reaches leave without touching the
+// patch.  Walking the rows and columns serially (a thread per row, an FP64
+// exponential per cell) took 4.2 ms of a 131x93 patch's 4.3 ms step.
 struct AbsorbConst {
   double xlo0, xlo1, dx0, dx1, gxlo0, gxlo1, gxhi0, gxhi1, w2, p0, T0, rho0;
 };
@@ -246,37 +295,89 @@ __device__ __forceinline__ void absorb_apply(PatchFields8 F, long g, double tmp,
   F.f[4][g] = relax_to(F.f[4][g], __dmul_rn(A.T0, A.rho0), tmp);
 }
 
-__global__ void absorb_kernel(PatchFields8 F, long pitch, int nx, int ny, int g0, int g1, int dir,
-                              AbsorbConst A) {
+__global__ void __launch_bounds__(256) absorb_kernel(PatchFields8 F, long pitch, int nx, int ny, int g0, int g1,
+                                                     int dirs, AbsorbConst A) {
+  // factor of the block's columns (L, R) and rows (B, T), and whether the
+  // walk from the side reaches them (2: only past the first row's test)
+  __shared__ double s_f[4][32];
+  __shared__ unsigned char s_r[4][32];
+  const int tid = threadIdx.x, i0 = blockIdx.x * 32, j0 = blockIdx.y * 8;
+  int any = 0;
+  if (tid < 128) {
+    const int dir = tid >> 5, q = tid & 31;
+    const int n = dir < 2 ? nx : ny, c = (dir < 2 ? i0 : j0) + q;
+    if ((dirs & (1 << dir)) && c < n && (dir < 2 || q < 8)) {
+      auto factor = [&](int m) {
+        if (dir < 2) {
+          const double xc = A.xlo0 + A.dx0 * ((double)m + 0.5);
+          return envelope(dir == 0 ? (xc - A.gxlo0) : (A.gxhi0 - xc), A.w2);
+        }
+        const double yc = A.xlo1 + A.dx1 * ((double)m + 0.5);
+        return envelope(dir == 2 ? (yc - A.gxlo1) : (A.gxhi1 - yc), A.w2);
+      };
+      auto go_on = [](double tmp) { return fabs(1.0 - tmp) > 1.0e-8; };
+      const bool first = c == ((dir & 1) ? n - 1 : 0);
+      const double f = factor(c);
+      // the edge cell itself is walked without a test in x, except on the
+      // first row, and with its own factor's test there and in y
+      int r = first ? (go_on(f) ? 1 : (dir < 2 ? 2 : 0)) : (go_on(factor((dir & 1) ? c + 1 : c - 1)) ? 1 : 0);
+      s_f[dir][q] = f;
+      s_r[dir][q] = (unsigned char)r;
+      any = r;
+    } else {
+      s_r[dir][q] = 0;
+    }
+  }
+  if (!__syncthreads_or(any)) return;
+  const int lx = tid & 31, ly = tid >> 5, ci = i0 + lx, cj = j0 + ly;
+  if (ci >= nx || cj >= ny) return;
+  int reach = 0;
+#pragma unroll
+  for (int dir = 0; dir < 4; ++dir) {
+    const int r = s_r[dir][dir < 2 ? lx : ly];
+    if (r == 1 || (r == 2 && cj != 0)) reach |= 1 << dir;
+  }
+  if (!reach) return;
+  const long g = (long)(cj + g1) * pitch + (ci + g0);
+  double v[7];
+#pragma unroll
+  for (int k = 0; k < 7; ++k) v[k] = F.f[k][g];
+  const double rT = __dmul_rn(A.T0, A.rho0);
+#pragma unroll
+  for (int dir = 0; dir < 4; ++dir) {
+    if (!(reach & (1 << dir))) continue;
+    const double tmp = s_f[dir][dir < 2 ? lx : ly];
+    v[5] = relax_to(v[5], A.p0, tmp);
+    v[6] = relax_to(v[6], A.T0, tmp);
+    v[0] = relax_to(v[0], A.rho0, tmp);
+    v[1] = __dmul_rn(v[1], tmp);
+    v[2] = __dmul_rn(v[2], tmp);
+    v[3] = __dmul_rn(v[3], tmp);
+    v[4] = relax_to(v[4], rT, tmp);
+  }
+#pragma unroll
+  for (int k = 0; k < 7; ++k) F.f[k][g] = v[k];
+}
+
+// The same walks serially, for a patch that lies partly outside the domain
+// (its distance from a side is not positive at the walk's first cell, so the
+// factors need not grow along the walk): one thread per row or column.
+__global__ void absorb_walk_kernel(PatchFields8 F, long pitch, int nx, int ny, int g0, int g1, int dir,
+                                   AbsorbConst A) {
   const double ep = 1.0e-8;
-  int t = blockIdx.x * blockDim.x + threadIdx.x;
-  if (dir < 2) {
-    if (t >= ny) return;
-    int cj = t;
-    double tmp;
-    auto xdist = [&](int ci) {
-      double xc = A.xlo0 + A.dx0 * ((double)ci + 0.5);
-      return dir == 0 ? (xc - A.gxlo0) : (A.gxhi0 - xc);
-    };
-    tmp = (cj == 0) ? envelope(xdist(dir == 0 ? 0 : nx - 1), A.w2) : 0.0;
-    for (int n = 0; (fabs(1.0 - tmp) > ep) && n < nx; ++n) {
-      int ci = dir == 0 ? n : nx - 1 - n;
-      tmp = envelope(xdist(ci), A.w2);
-      absorb_apply(F, (long)(cj + g1) * pitch + (ci + g0), tmp, A);
-    }
-  } else {
-    if (t >= nx) return;
-    int ci = t;
-    auto ydist = [&](int cj) {
-      double yc = A.xlo1 + A.dx1 * ((double)cj + 0.5);
-      return dir == 2 ? (yc - A.gxlo1) : (A.gxhi1 - yc);
-    };
-    double tmp = envelope(ydist(dir == 2 ? 0 : ny - 1), A.w2);
-    for (int n = 0; (fabs(1.0 - tmp) > ep) && n < ny; ++n) {
-      int cj = dir == 2 ? n : ny - 1 - n;
-      tmp = envelope(ydist(cj), A.w2);
-      absorb_apply(F, (long)(cj + g1) * pitch + (ci + g0), tmp, A);
-    }
+  const int t = blockIdx.x * blockDim.x + threadIdx.x;
+  const bool x = dir < 2;
+  if (t >= (x ? ny : nx)) return;
+  const int len = x ? nx : ny;
+  auto dist = [&](int c) {
+    const double q = x ? A.xlo0 + A.dx0 * ((double)c + 0.5) : A.xlo1 + A.dx1 * ((double)c + 0.5);
+    return (dir & 1) ? ((x ? A.gxhi0 : A.gxhi1) - q) : (q - (x ? A.gxlo0 : A.gxlo1));
+  };
+  double tmp = (!x || t == 0) ? envelope(dist((dir & 1) ? len - 1 : 0), A.w2) : 0.0;
+  for (int n = 0; (fabs(1.0 - tmp) > ep) && n < len; ++n) {
+    const int c = (dir & 1) ? len - 1 - n : n;
+    tmp = envelope(dist(c), A.w2);
+    absorb_apply(F, x ? (long)(t + g1) * pitch + (c + g0) : (long)(c + g1) * pitch + (t + g0), tmp, A);
   }
 }
 
@@ -450,10 +551,9 @@ void runge_kutta_(const int& ifirst0, const int& ilast0, const int& ifirst1, con
     return;
   }
   long pitch = nx + 2 * gcw0, fstride = pitch * (ny + 2 * gcw1);
-  dim3 block(32, 4);
-  runge_kutta_kernel<<<grid2d(nx, ny, block), block, 0, stream()>>>(
-      w_n, pitch, fstride, gcw0, gcw1, w, rhs, nx, (long)nx * ny, nx, ny, nequ, alpha_1, alpha_2,
-      beta * dt);
+  const dim3 block(32, 4), grid((nx + 32 * kRkCells - 1) / (32 * kRkCells), (ny + 3) / 4, nequ);
+  runge_kutta_kernel<<<grid, block, 0, stream()>>>(w_n, pitch, fstride, gcw0, gcw1, w, rhs, nx, (long)nx * ny, nx, ny,
+                                                   alpha_1, alpha_2, beta * dt);
   check_launch("runge_kutta");
 }
 
@@ -508,28 +608,36 @@ int enl_phys_bc(int ifirst0, int ilast0, int ifirst1, int ilast1, int gcw0, int 
     return ENL_ERR_ARG;
   }
   long pitch = nx + 2 * gcw0, fstride = pitch * (ny + 2 * gcw1);
-  PatchFields8 F;
-  for (int k = 0; k < 5; ++k) F.f[k] = w_n + k * fstride;
-  F.f[5] = pressure;
-  F.f[6] = temperature;
-  F.f[7] = source;
-  cudaStream_t s = stream();
+  BandArgs A;
+  for (int k = 0; k < 5; ++k) A.F.f[k] = w_n + k * fstride;
+  A.F.f[5] = pressure;
+  A.F.f[6] = temperature;
+  A.F.f[7] = source;
+  A.pitch = pitch;
+  A.nx = nx;
+  A.ny = ny;
+  A.g0 = gcw0;
+  A.g1 = gcw1;
+  A.fill0 = fill0;
+  A.fill1 = fill1;
+  A.touches = A.reflect = 0;
+  long cells = 0;
   for (int side = 0; side < 4; ++side) {
-    if (!touches[side]) continue;
-    int fill = side < 2 ? fill0 : fill1;
-    int n = ((side < 2) ? ny : nx) * fill * 8;
-    if (n == 0) continue;
-    phys_bc_edge_kernel<<<(n + 127) / 128, 128, 0, s>>>(F, pitch, nx, ny, gcw0, gcw1, side, fill,
-                                                        bc[side] == kReflect);
+    if (touches[side]) {
+      A.touches |= 1 << side;
+      cells += side < 2 ? (long)ny * fill0 : (long)nx * fill1;
+    }
+    if (bc[side] == kReflect) A.reflect |= 1 << side;
   }
-  for (int loc = 0; loc < 4; ++loc) {
-    int xs = loc & 1, ys = (loc >> 1) & 1;
-    if (!(touches[xs ? 1 : 0] || touches[ys ? 3 : 2])) continue;
-    int n = fill0 * fill1 * 8;
-    if (n == 0) continue;
-    phys_bc_node_kernel<<<(n + 127) / 128, 128, 0, s>>>(F, pitch, nx, ny, gcw0, gcw1, loc, fill0, fill1,
-                                                        bc[xs ? 1 : 0] == kReflect);
+  for (int loc = 0; loc < 4; ++loc)
+    if (touches[loc & 1] || touches[2 + (loc >> 1)]) cells += (long)fill0 * fill1;
+  if (cells == 0) return ENL_OK;
+  if (cells > INT_MAX / 2) {
+    set_error(ENL_ERR_ARG);
+    return ENL_ERR_ARG;
   }
+  A.cells = (int)cells;
+  phys_bc_kernel<<<dim3((unsigned)std::min<long>((cells + 127) / 128, 4096), 8), 128, 0, stream()>>>(A);
   return check_launch("phys_bc");
 }
 
@@ -552,11 +660,23 @@ int enl_absorb(int ifirst0, int ilast0, int ifirst1, int ilast1, int gcw0, int g
   F.f[7] = nullptr;
   AbsorbConst A{patch_xlo[0], patch_xlo[1], dx[0], dx[1], grid_xlo[0], grid_xlo[1], grid_xhi[0], grid_xhi[1],
                 absorb_width * absorb_width, p0, T0, rho0};
-  cudaStream_t s = stream();
-  for (int dir = 0; dir < 4; ++dir) {
-    if (bc[dir] != kAbsorb) continue;
-    int n = dir < 2 ? ny : nx;
-    absorb_kernel<<<(n + 127) / 128, 128, 0, s>>>(F, pitch, nx, ny, gcw0, gcw1, dir, A);
+  // distance of each walk's first cell from its side
+  const double first[4] = {(A.xlo0 + A.dx0 * 0.5) - A.gxlo0, A.gxhi0 - (A.xlo0 + A.dx0 * (nx - 0.5)),
+                           (A.xlo1 + A.dx1 * 0.5) - A.gxlo1, A.gxhi1 - (A.xlo1 + A.dx1 * (ny - 0.5))};
+  int dirs = 0;
+  bool inside = A.dx0 > 0.0 && A.dx1 > 0.0 && A.w2 > 0.0;
+  for (int dir = 0; dir < 4; ++dir)
+    if (bc[dir] == kAbsorb) {
+      dirs |= 1 << dir;
+      inside = inside && first[dir] > 0.0;
+    }
+  if (inside) {
+    absorb_kernel<<<dim3((nx + 31) / 32, (ny + 7) / 8), 256, 0, stream()>>>(F, pitch, nx, ny, gcw0, gcw1, dirs, A);
+  } else {
+    for (int dir = 0; dir < 4; ++dir)
+      if (dirs & (1 << dir))
+        absorb_walk_kernel<<<((dir < 2 ? ny : nx) + 127) / 128, 128, 0, stream()>>>(F, pitch, nx, ny, gcw0, gcw1, dir,
+                                                                                    A);
   }
   return check_launch("absorb");
 }
