@@ -14,69 +14,17 @@
 //   * velocities and fluxes come from the planes (a cell used to divide 23
 //     times);
 //   * the hybrid switch decides bit for bit as the reference's division
-//     would (sensor_line_fast), dividing only ratios that lie within 2^-44 of
+//     would (enl_ratio.cuh), in single precision unless a ratio lies close to
 //     the threshold.
 // Results stay within rounding of the reference's (the engine is held to the
 // oracle at 1e-12 relative L2 per field).
 #pragma once
+#include "enl_eos.cuh"
 #include "enl_fast.cuh"
+#include "enl_ratio.cuh"
 #include "enl_triple.cuh"
 
 namespace enl {
-
-// Reciprocal of a double.  For positive normal x within the float exponent
-// range, the double's exponent and top 20 mantissa bits are moved into a
-// float by integer operations, the hardware single-precision reciprocal gives
-// a seed r with |1 - x r| < 2^-19, and one Newton step with its cubic term,
-// r (1 + e + e^2) with e = 1 - x r, leaves |1 - x r'| = |e|^3 < 2^-57, below
-// FP64 rounding.  Zero, negative, non-finite and out-of-range arguments take
-// the division.  All bit manipulation is on unsigned integers, so no shift
-// overflows.
-__device__ __forceinline__ double rcp64(double x) {
-  const unsigned hi = (unsigned)__double2hiint(x);
-  const unsigned e = hi >> 20;  // sign and biased exponent
-  if (e - (1023u - 125u) > 250u) return 1.0 / x;
-  const float xf = __uint_as_float((hi - ((1023u - 127u) << 20)) << 3);
-  const unsigned rb = __float_as_uint(rcp_approx(xf));
-  const double r = __hiloint2double((int)((rb >> 3) + ((1023u - 127u) << 20)), (int)(rb << 29));
-  const double ee = fma(-x, r, 1.0);
-  return fma(r, fma(ee, ee, ee), r);
-}
-
-// The hybrid switch of rhs_hybrid_high_llf.m4:239-256 along one direction,
-// r[0..4] = rho at offsets -2..2; the same decision as sensor_line_exact bit
-// for bit.  Each ratio num / den (both >= ep > 0, rounded as the reference
-// rounds them) is first estimated as num * rcp64(den), within 2^-50 of the
-// exact quotient; the reference's correctly rounded quotient is below the
-// threshold c when the estimate is below c (1 - 2^-44) and not below it when
-// the estimate is above c (1 + 2^-44).  Only ratios in between are divided.
-// Two zero differences give num = den = ep, a ratio of 1: no WENO.
-__device__ __forceinline__ int sensor_line_fast(const double r[5], double ep) {
-  constexpr double kLo = Lit::c0_9999 * (1.0 - 0x1p-44);
-  constexpr double kHi = Lit::c0_9999 * (1.0 + 0x1p-44);
-  double t[4], sq[4];
-#pragma unroll
-  for (int q = 0; q < 4; ++q) {
-    t[q] = __dsub_rn(r[q + 1], r[q]);
-    sq[q] = __dmul_rn(t[q], t[q]);
-  }
-  int tag = 0;
-#pragma unroll
-  for (int q = 0; q < 3; ++q) {
-    const double t1 = t[q], t2 = t[q + 1];
-    const unsigned long long mag =
-        ((unsigned long long)__double_as_longlong(t1) | (unsigned long long)__double_as_longlong(t2)) << 1;
-    if (mag != 0ull) {  // (both differences zero, of either sign: ratio 1)
-      const double num = __dadd_rn(__dmul_rn(2.0, fabs(__dmul_rn(t1, t2))), ep);
-      const double den = __dadd_rn(__dadd_rn(sq[q], sq[q + 1]), ep);
-      // positive quotient: its bit pattern orders as its value
-      const unsigned long long qb = (unsigned long long)__double_as_longlong(num * rcp64(den));
-      if (qb < (unsigned long long)__double_as_longlong(kLo)) tag = 1;
-      else if (qb <= (unsigned long long)__double_as_longlong(kHi) && __ddiv_rn(num, den) < Lit::c0_9999) tag = 1;
-    }
-  }
-  return tag;
-}
 
 // FP64 planes of a 38 x (TH + 6) halo tile (rows of kBW64 doubles; TH = 8 in
 // the batched engine): u and v at every position, the half fluxes F_0..4 / 2
@@ -157,10 +105,10 @@ __device__ __forceinline__ int switch64(const SAcc64P<TH>& A, const RhsConst& P)
   double r[5];
 #pragma unroll
   for (int q = 0; q < 5; ++q) r[q] = A.w(0, q - 2, 0);
-  int tag = sensor_line_fast(r, P.sensor_eps);
+  int tag = sensor_line(r, P.sensor_eps, P.sensor_eps32);
 #pragma unroll
   for (int q = 0; q < 5; ++q) r[q] = A.w(0, 0, q - 2);
-  return tag | sensor_line_fast(r, P.sensor_eps);
+  return tag || sensor_line(r, P.sensor_eps, P.sensor_eps32);
 }
 
 // Viscous, entropy-production and relaxation sources H1..H4
@@ -199,7 +147,7 @@ __device__ __forceinline__ void sources64(const SAcc64P<TH>& A, const RhsConst& 
   double Mn = (Tc - T_n) * P.inv_tau_n;
   double inv_Tn = rcp64(T_n);
   double tmp1 = P.T_star_n * inv_Tn;
-  double c_vn = ((Lit::c0_78 * P.R) * (tmp1 * tmp1)) * exp(-tmp1);
+  double c_vn = ((Lit::c0_78 * P.R) * (tmp1 * tmp1)) * (fabs(tmp1) < 700.0 ? exp64(-tmp1) : exp(-tmp1));
   double A_n = (Tc * inv_Tn - 1.0) * c_vn;
   double phi_xx = c43 * ux - c23 * vy;
   double phi_xy = uy + vx;

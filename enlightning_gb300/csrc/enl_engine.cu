@@ -186,44 +186,7 @@ __device__ __forceinline__ double relax_(double q, double amb, double tmp) {
   return __dadd_rn(__dmul_rn(__dsub_rn(q, amb), tmp), amb);
 }
 
-// update_state (update_state.m4:90-105) on absolute FP64 values, with the
-// reference's rounding; height = centre height of the cell row.
-struct EosConst64 {
-  double rho0, c, c_lr, gm1_over_2rho0, c_p, p0, T0, c_v, R;
-  double inv_c_p, inv_c_v;  // 1/c_p, 1/c_v (eos_fast64)
-};
-__device__ __forceinline__ void eos_abs64(const EosConst64& E, double w0, double w3, double height, double& p,
-                                          double& T) {
-  const double cc = __dadd_rn(E.c, __dmul_rn(E.c_lr, height));
-  const double d = __dsub_rn(w0, E.rho0);
-  const double s = __ddiv_rn(w3, w0);
-  const double inner =
-      __dadd_rn(__dadd_rn(d, __dmul_rn(E.gm1_over_2rho0, __dmul_rn(d, d))), __dmul_rn(__ddiv_rn(w0, E.c_p), s));
-  p = __dadd_rn(__dmul_rn(__dmul_rn(cc, cc), inner), E.p0);
-  T = E.T0 * exp((s - E.R * log(E.rho0 / w0)) / E.c_v);
-}
-
-// The same as the batched FP64 engine computes it (stage epilogue and state
-// upload alike, so the two agree bit for bit): one seeded reciprocal of rho
-// (rcp64) instead of two divisions, constant divisors as factors, every
-// operation explicitly rounded (no contraction differences between call
-// sites).  Within a few units in the last place of eos_abs64.
-__device__ __forceinline__ double row_height64(double ylo, double dy, int j) {
-  return __dadd_rn(ylo, __dmul_rn(dy, (double)j + 0.5));
-}
-__device__ __forceinline__ void eos_fast64(const EosConst64& E, double w0, double w3, double height, double& p,
-                                           double& T) {
-  const double cc = __dadd_rn(E.c, __dmul_rn(E.c_lr, height));
-  const double ir = rcp64(w0);
-  const double d = __dsub_rn(w0, E.rho0);
-  const double s = __dmul_rn(w3, ir);
-  const double inner =
-      __dadd_rn(__dadd_rn(d, __dmul_rn(E.gm1_over_2rho0, __dmul_rn(d, d))), __dmul_rn(__dmul_rn(w0, E.inv_c_p), s));
-  p = __dadd_rn(__dmul_rn(__dmul_rn(cc, cc), inner), E.p0);
-  T = __dmul_rn(E.T0, exp(__dmul_rn(__dsub_rn(s, __dmul_rn(E.R, log(__dmul_rn(E.rho0, ir)))), E.inv_c_v)));
-}
-
-// The same in single-precision perturbation form: rp = rho - rho0, w3 = rho s;
+// update_state (update_state.m4:90-105) in single-precision perturbation form: rp = rho - rho0, w3 = rho s;
 // returns p - p0 and T - T0 (log1p/expm1 keep small perturbations exact).
 struct EosConst32 {
   float rho0, c, c_lr, gm1_over_2rho0, inv_c_p, T0, inv_c_v, R, inv_rho0;
@@ -1142,7 +1105,7 @@ __global__ void __launch_bounds__(256, std::is_same<S, float>::value ? kStageBlo
               wn[k] = (A.a1 * un[k * fs + g] + A.a2 * win) + bdt * (H[k] - D[k]);
             }
             // update_state (update_state.m4:90-105), as the state upload computes it
-            eos_fast64(A.E64, wn[0], wn[3], row_height64(A.ylo, A.dy[lvl], gj), pv, tv);
+            eos64(A.E64, wn[0], wn[3], row_height64(A.ylo, A.dy[lvl], gj), pv, tv);
           }
           if (s_tile.absorb) {  // absolute values relax towards the ambient state
             const int reach = absorb_reach(A.absorb, lvl, gi, gj, s_tile.box, s_tile.absorb);
@@ -1508,31 +1471,7 @@ __global__ void refine_box_kernel(CanvasT<S> F, CanvasT<S> C, int ratio, const i
 }
 
 // tag_cells.m4:58-108 over the tiles of one level, bit-exact.
-// Decided bit for bit as the reference's division would, with the estimate
-// of the hybrid switch (sensor_line_fast): two zero differences give the
-// ratio ep / ep, 1 or NaN, never below the threshold (most cells of a mostly
-// quiet level); otherwise, for a tolerance ep above 2^-1000 (num and den are
-// then normal, at least ep), an estimate num * rcp64(den) within 2^-50 of the
-// quotient decides unless it lies within 2^-44 of the threshold, and only
-// those ratios are divided.
-__device__ __forceinline__ bool ratio_below_e(double fm, double f0, double fp, double ep) {
-  constexpr double kLo = Lit::c0_9999 * (1.0 - 0x1p-44);
-  constexpr double kHi = Lit::c0_9999 * (1.0 + 0x1p-44);
-  const double t1 = __dsub_rn(f0, fm);
-  const double t2 = __dsub_rn(fp, f0);
-  const unsigned long long mag =
-      ((unsigned long long)__double_as_longlong(t1) | (unsigned long long)__double_as_longlong(t2)) << 1;
-  if (mag == 0ull) return false;
-  const double num = __dadd_rn(__dmul_rn(2.0, fabs(__dmul_rn(t1, t2))), ep);
-  const double den = __dadd_rn(__dadd_rn(__dmul_rn(t1, t1), __dmul_rn(t2, t2)), ep);
-  if (!(ep > 0x1p-1000)) return __ddiv_rn(num, den) < Lit::c0_9999;
-  // a positive quotient (or NaN, whose pattern is above kHi): its bit
-  // pattern orders as its value
-  const unsigned long long qb = (unsigned long long)__double_as_longlong(num * rcp64(den));
-  if (qb < (unsigned long long)__double_as_longlong(kLo)) return true;
-  return qb <= (unsigned long long)__double_as_longlong(kHi) && __ddiv_rn(num, den) < Lit::c0_9999;
-}
-
+// (enl_ratio.cuh.)
 // The same test in single precision for FP32 storage (FP64 division is slow
 // on this part and the fast engine's tags need no bit-exactness); 0.9999f is
 // the reference's REAL*4 literal itself.
@@ -1550,8 +1489,8 @@ template <typename S>
 // the tagged cells as bits of per-block words (block B x B cells, bit
 // r*B + c for cell (c, r) of the block, B <= 8; the words zeroed before).
 __global__ void tag_tiles_kernel(int* tags, CanvasT<S> W, CanvasT<S> H, const int4* tiles, int off, int cnt,
-                                 double ep0, double ep1, unsigned long long* mask = nullptr, int B = 1,
-                                 int nbx = 0) {
+                                 double ep0, float ep0f, double ep1, float ep1f, unsigned long long* mask = nullptr,
+                                 int B = 1, int nbx = 0) {
   for (int t = blockIdx.x; t < cnt; t += gridDim.x) {
     int4 td = tiles[off + t];
     int w = (td.z >> 8) & 0xff, h = (td.z >> 16) & 0xff;
@@ -1566,10 +1505,7 @@ __global__ void tag_tiles_kernel(int* tags, CanvasT<S> W, CanvasT<S> H, const in
            ratio_below_f(W.at(0, i - 1, j), W.at(0, i, j), W.at(0, i + 1, j), e1) ||
            ratio_below_f(W.at(0, i, j - 1), W.at(0, i, j), W.at(0, i, j + 1), e1);
     } else {
-      tg = ratio_below_e(H.at(0, i - 1, j), H.at(0, i, j), H.at(0, i + 1, j), ep0) ||
-           ratio_below_e(H.at(0, i, j - 1), H.at(0, i, j), H.at(0, i, j + 1), ep0) ||
-           ratio_below_e(W.at(0, i - 1, j), W.at(0, i, j), W.at(0, i + 1, j), ep1) ||
-           ratio_below_e(W.at(0, i, j - 1), W.at(0, i, j), W.at(0, i, j + 1), ep1);
+      tg = tag_cell64(&H.at(0, i, j), &W.at(0, i, j), W.pitch, ep0, ep0f, ep1, ep1f);
     }
     if (tags) tags[(long)j * W.nx + i] = tg ? 1 : 0;
     if (mask && tg) {
@@ -1629,20 +1565,15 @@ __global__ void rk_plain_kernel(CanvasView S, CanvasView U, CanvasView K, int il
                               __dmul_rn(bdt, K.at(k, i, j)));
 }
 
-struct EosArgs {
-  double rho0, c, gm1_over_2rho0, c_p, p0, T0, c_lr, c_v, R, ylo, dy;
-};
-
-__global__ void eos_plain_kernel(CanvasView S, int ilo, int jlo, int w, int h, EosArgs E) {
+__global__ void eos_plain_kernel(CanvasView S, int ilo, int jlo, int w, int h, double ylo, double dy,
+                                 const __grid_constant__ EosConst64 E) {
   int ci = blockIdx.x * blockDim.x + threadIdx.x, cj = blockIdx.y * blockDim.y + threadIdx.y;
   if (ci >= w || cj >= h) return;
   int i = ilo + ci, j = jlo + cj;
   // update_state.m4:88 uses the patch's xlo and (j - ifirst1); with the level
   // origin that is the same centre height.
-  const double height = __dadd_rn(E.ylo, __dmul_rn(E.dy, (double)j + 0.5));
-  const EosConst64 K{E.rho0, E.c, E.c_lr, E.gm1_over_2rho0, E.c_p, E.p0, E.T0, E.c_v, E.R, 1.0 / E.c_p, 1.0 / E.c_v};
   double p, T;
-  eos_abs64(K, S.at(0, i, j), S.at(3, i, j), height, p, T);
+  eos64(E, S.at(0, i, j), S.at(3, i, j), row_height64(ylo, dy, j), p, T);
   S.at(5, i, j) = p;
   S.at(6, i, j) = T;
 }
@@ -2117,7 +2048,7 @@ __global__ void pack_kernel(PackArgs<S> A) {
           V.at(6, i, j) = tp;
         } else {
           double pv, tv;
-          eos_fast64(A.E64, v[0], v[3], row_height64(A.ylo, A.dy[lvl], j), pv, tv);
+          eos64(A.E64, v[0], v[3], row_height64(A.ylo, A.dy[lvl], j), pv, tv);
           V.at(5, i, j) = pv;
           V.at(6, i, j) = tv;
         }
@@ -2838,8 +2769,7 @@ static EosConst32 eos_const32(const enl_engine_config& c) {
 }
 
 static EosConst64 eos_const64(const enl_engine_config& c) {
-  return EosConst64{c.rho0, c.c, c.c_lr, (c.gamma1 - 1.0) / (2.0 * c.rho0), c.c_p, c.p0, c.T0, c.c_v, c.R,
-                    1.0 / c.c_p, 1.0 / c.c_v};
+  return make_eos_const64(c.rho0, c.c, c.c_lr, c.gamma1, c.c_p, c.p0, c.T0, c.c_v, c.R);
 }
 
 // level < 0: the launch covers every tile of every level; otherwise the
@@ -3358,8 +3288,7 @@ static int step_plain(Engine* E, double dt) {
     }
     for (int l = 0; l < nl; ++l) {
       Level& L = E->lev[l];
-      EosArgs Ea{c.rho0, c.c, (c.gamma1 - 1.0) / (2.0 * c.rho0), c.c_p, c.p0, c.T0, c.c_lr, c.c_v, c.R, c.xlo[1],
-                 L.dx[1]};
+      const EosConst64 Ec = eos_const64(c);
       CanvasView K{L.kk, L.pitch, L.fstride, L.nx, L.ny};
       for (auto& b : L.patches) {
         int nx = b.y - b.x + 1, ny = b.w - b.z + 1;
@@ -3367,7 +3296,7 @@ static int step_plain(Engine* E, double dt) {
         rk_plain_kernel<<<grd, blk, 0, s>>>(L.view<double>(1), L.view<double>(0), K, b.x, b.z, nx, ny,
                                             c.rk_alpha1[st], c.rk_alpha2[st], c.rk_beta[st] * dt, c.rk_beta[st],
                                             E->adaptive ? E->d_dt : nullptr);
-        eos_plain_kernel<<<grd, blk, 0, s>>>(L.view<double>(1), b.x, b.z, nx, ny, Ea);
+        eos_plain_kernel<<<grd, blk, 0, s>>>(L.view<double>(1), b.x, b.z, nx, ny, c.xlo[1], L.dx[1], Ec);
       }
     }
     absorb_all(E, 1);
@@ -3802,11 +3731,13 @@ static int tag_level(Engine* E, int level, int* tags, unsigned long long* mask, 
     if (E->f32s)
       tag_tiles_kernel<float><<<E->tile_cnt[level], 256, 0, s>>>(tags, L.view<float>(0), L.view<float>(3),
                                                                  E->d_tiles.p, E->tile_off[level],
-                                                                 E->tile_cnt[level], ep0, ep1, mask, B, nbx);
+                                                                 E->tile_cnt[level], ep0, ratio_eps32(ep0), ep1,
+                                                                  ratio_eps32(ep1), mask, B, nbx);
     else
       tag_tiles_kernel<double><<<E->tile_cnt[level], 256, 0, s>>>(tags, L.view<double>(0), L.view<double>(3),
                                                                   E->d_tiles.p, E->tile_off[level],
-                                                                  E->tile_cnt[level], ep0, ep1, mask, B, nbx);
+                                                                  E->tile_cnt[level], ep0, ratio_eps32(ep0), ep1,
+                                                                  ratio_eps32(ep1), mask, B, nbx);
   return check_launch("engine tag");
 }
 

@@ -16,17 +16,9 @@
 // them instead of recomputing them for every stencil point.
 #pragma once
 #include "enl_physics.cuh"
+#include "enl_rcp.cuh"
 
 namespace enl {
-
-// Single-precision reciprocal of the hardware (rcp.approx, within 1 ulp);
-// every use is inside the FP32 perturbation path, whose error budget is
-// orders of magnitude above that.
-__device__ __forceinline__ float rcp_approx(float x) {
-  float r;
-  asm("rcp.approx.ftz.f32 %0, %1;" : "=f"(r) : "f"(x));
-  return r;
-}
 
 struct FastConst {
   float inv_dx0, inv_dx1, inv_dx0sq, inv_dx1sq, inv_2dx0, inv_2dx1, inv_4dxdy;

@@ -132,54 +132,29 @@ __global__ void __launch_bounds__(128) runge_kutta_kernel(double* __restrict__ w
   }
 }
 
-struct StateConst {
-  double rho0, c, gm1_over_2rho0, c_p, p0, T0, c_lr, c_v, R, ylo, dy;
-};
-
-// update_state.m4:87-107.
-__device__ __forceinline__ void eos_f64(double w0, double w3, double height, const StateConst& S, double& p,
-                                        double& T) {
-  double cc = __dadd_rn(S.c, __dmul_rn(S.c_lr, height));
-  double d = __dsub_rn(w0, S.rho0);
-  double s = __ddiv_rn(w3, w0);
-  double inner = __dadd_rn(__dadd_rn(d, __dmul_rn(S.gm1_over_2rho0, __dmul_rn(d, d))), __dmul_rn(__ddiv_rn(w0, S.c_p), s));
-  p = __dadd_rn(__dmul_rn(__dmul_rn(cc, cc), inner), S.p0);
-  T = S.T0 * exp((s - S.R * log(S.rho0 / w0)) / S.c_v);
-}
-
+// update_state.m4:87-107 (eos64).
 __global__ void update_state_kernel(const double* __restrict__ w, double* __restrict__ pres,
                                     double* __restrict__ temp, long pitch, long fstride, int g0, int g1,
-                                    int nx, int ny, StateConst S) {
+                                    int nx, int ny, double ylo, double dy, const __grid_constant__ EosConst64 E) {
   int ci = blockIdx.x * blockDim.x + threadIdx.x;
   int cj = blockIdx.y * blockDim.y + threadIdx.y;
   if (ci >= nx || cj >= ny) return;
   long g = (long)(cj + g1) * pitch + (ci + g0);
-  double height = __dadd_rn(S.ylo, __dmul_rn(S.dy, (double)cj + 0.5));
   double p, T;
-  eos_f64(w[g], w[3 * fstride + g], height, S, p, T);
+  eos64(E, w[g], w[3 * fstride + g], row_height64(ylo, dy, cj), p, T);
   pres[g] = p;
   temp[g] = T;
 }
 
-// tag_cells.m4:58-108, bit-exact (explicitly rounded operations).
-__device__ __forceinline__ bool ratio_below(double fm, double f0, double fp, double ep) {
-  double t1 = __dsub_rn(f0, fm);
-  double t2 = __dsub_rn(fp, f0);
-  double num = __dadd_rn(__dmul_rn(2.0, fabs(__dmul_rn(t1, t2))), ep);
-  double den = __dadd_rn(__dadd_rn(__dmul_rn(t1, t1), __dmul_rn(t2, t2)), ep);
-  return __ddiv_rn(num, den) < Lit::c0_9999;
-}
-
+// tag_cells.m4:58-108, bit-exact (enl_ratio.cuh).
 __global__ void tag_cells_kernel(int* __restrict__ tags, long tpitch, const double* __restrict__ w,
                                  const double* __restrict__ H0, long pitch, int g0, int g1, int nx, int ny,
-                                 int tag_val, double ep0, double ep1) {
+                                 int tag_val, double ep0, float ep0f, double ep1, float ep1f) {
   int ci = blockIdx.x * blockDim.x + threadIdx.x;
   int cj = blockIdx.y * blockDim.y + threadIdx.y;
   if (ci >= nx || cj >= ny) return;
   long g = (long)(cj + g1) * pitch + (ci + g0);
-  bool t = ratio_below(H0[g - 1], H0[g], H0[g + 1], ep0) || ratio_below(H0[g - pitch], H0[g], H0[g + pitch], ep0) ||
-           ratio_below(w[g - 1], w[g], w[g + 1], ep1) || ratio_below(w[g - pitch], w[g], w[g + pitch], ep1);
-  tags[(long)cj * tpitch + ci] = t ? tag_val : 0;
+  tags[(long)cj * tpitch + ci] = tag_cell64(H0 + g, w + g, pitch, ep0, ep0f, ep1, ep1f) ? tag_val : 0;
 }
 
 // Physical-boundary fill, enlightning.C:830-1008.  Each ghost cell of an edge
@@ -412,6 +387,7 @@ RhsConst make_rhs_const(const double* xlo, const double* dx, double alpha, doubl
   // contraction of host code so the value is the reference's.
   const double xi = 1.0;
   P.sensor_eps = ((Lit::c0_9 * tol[2]) * (xi * xi)) / (1.0 - Lit::c0_9 * (tol[2] * tol[2]));
+  P.sensor_eps32 = ratio_eps32(P.sensor_eps);
   P.level = level;
   return P;
 }
@@ -572,10 +548,10 @@ void update_state_(const double* dx, const double* xlo, const int& ifirst0, cons
     return;
   }
   long pitch = nx + 2 * gcw0, fstride = pitch * (ny + 2 * gcw1);
-  StateConst S{rho0, c, (gamma1 - 1.0) / (2.0 * rho0), c_p, p0, T0, c_lr, c_v, R, xlo[1], dx[1]};
+  const EosConst64 E = make_eos_const64(rho0, c, c_lr, gamma1, c_p, p0, T0, c_v, R);
   dim3 block(32, 4);
   update_state_kernel<<<grid2d(nx, ny, block), block, 0, stream()>>>(w_n, pressure, temperature, pitch,
-                                                                       fstride, gcw0, gcw1, nx, ny, S);
+                                                                       fstride, gcw0, gcw1, nx, ny, xlo[1], dx[1], E);
   check_launch("update_state");
 }
 
@@ -594,7 +570,8 @@ void tag_cells_(const int& ifirst0, const int& ilast0, const int& ifirst1, const
   double ep1 = ((Lit::c0_9 * tag_tolerance[1]) * (xi * xi)) / (1.0 - Lit::c0_9 * (tag_tolerance[1] * tag_tolerance[1]));
   dim3 block(32, 4);
   tag_cells_kernel<<<grid2d(nx, ny, block), block, 0, stream()>>>(tags, nx, w_n, source, pitch, gcw0, gcw1, nx,
-                                                                    ny, refine_tag_val, ep0, ep1);
+                                                                  ny, refine_tag_val, ep0, ratio_eps32(ep0), ep1,
+                                                                  ratio_eps32(ep1));
   check_launch("tag_cells");
 }
 

@@ -28,6 +28,7 @@ struct RhsConst {
   double c, c_lr;                   // sound speed and lapse rate
   double ylo, dy;                   // height of row j: ylo + dy*((j - jfirst) + 0.5)
   double sensor_eps;                // ep of the hybrid sensor (tolerance(2))
+  float sensor_eps32;               // ratio_eps32 of it
   int level;
 };
 

@@ -39,7 +39,7 @@
 // them exactly, scaled by the largest one's power of two, so that no value of
 // the state overflows or underflows the single-precision range.
 #pragma once
-#include "enl_common.cuh"
+#include "enl_rcp.cuh"
 
 namespace enl {
 
@@ -133,11 +133,6 @@ __device__ __forceinline__ T3 t3_mul_f(T3 a, f2 c) {
   return T3{p, s, f2_fma(c, a.l, f2_add(f, r))};
 }
 
-__device__ __forceinline__ float rcp_seed(float x) {
-  float r;
-  asm("rcp.approx.ftz.f32 %0, %1;" : "=f"(r) : "f"(x));
-  return r;
-}
 // K / q for q > 0 normal, K a power of two.  One Newton step makes the
 // hardware seed y accurate to half a unit, so that the residual 1 - q.h y is
 // exact; then 1 / q = y (1 + r + r^2) with r = 1 - q y, |r| < 2^-21, whose
@@ -146,7 +141,7 @@ __device__ __forceinline__ T3 t3_rcp(T3 q, f2 K) {
   float a, b;
   f2_unpack(q.h, a, b);
   const f2 nq = f2_neg(q.h), nm = f2_neg(q.m), one = f2_both(1.f);
-  f2 y = f2_pack(rcp_seed(a), rcp_seed(b));
+  f2 y = f2_pack(rcp_approx(a), rcp_approx(b));
   y = f2_fma(y, f2_fma(nq, y, one), y);
   const f2 r = f2_fma(nq, y, one), p = f2_mul(nm, y), ep = f2_fma(nm, y, f2_neg(p));
   f2 rs, re;
