@@ -62,36 +62,50 @@ __device__ __forceinline__ SAcc64P<TH> acc64p(const double* t, const double* pl,
   return SAcc64P<TH>{t, pl, (cy + 3) * kBW64 + cx + 3, cy * kBW64 + cx + 3, (cy + 3) * 32 + cx};
 }
 
+// x / 2 by the exponent, on the integer pipe (zeros and normal results; the
+// others by the multiplication).
+__device__ __forceinline__ double half64(double x) {
+  const int hi = __double2hiint(x);
+  const unsigned e = (unsigned)hi & 0x7ff00000u;
+  if (e - 0x00200000u < 0x7fd00000u) return __hiloint2double(hi - 0x00100000, __double2loint(x));
+  if ((((unsigned)hi << 1) | (unsigned)__double2loint(x)) == 0u) return x;
+  return 0.5 * x;
+}
+
 // The planes of a tile of w x h cells from its staged box, by the whole block
 // of 256 threads (no barrier inside).  One seeded reciprocal of rho per halo
-// position; the flux planes hold half fluxes, formed from u/2, v/2 and p/2
-// (halving is exact, so each is F/2 or G/2 of the same double).  The
-// positions past a multiple of 256 fall on the last warp, not on warp 0, which
-// also stages the engine's next tile.
+// position; the flux planes hold half fluxes (halving is exact).  F_0 = rho u
+// and G_0 = rho v are state fields, F_2 = G_1 = rho u v.  The positions past a
+// multiple of 256 fall on the last warp, not on warp 0, which also stages the
+// engine's next tile.
 template <int TH>
 __device__ __forceinline__ void build_planes64(const double* tile, double* pl, int w, int h) {
   using G = Geo64<TH>;
   for (int e = 255 - (int)threadIdx.x; e < G::Pos; e += 256) {
     const int row = e / kBW64, col = e - row * kBW64;
     if (row >= h + 6 || col >= w + 6) continue;  // beyond a ragged tile
+    const double w1 = tile[G::Pos + e], w2 = tile[2 * G::Pos + e];
     const double ir = rcp64(tile[e]);
-    const double u = tile[G::Pos + e] * ir, v = tile[2 * G::Pos + e] * ir;
-    const double hp = 0.5 * tile[5 * G::Pos + e];
+    const double u = w1 * ir, v = w2 * ir, hu = half64(u), hv = half64(v);
+    const double hp = half64(tile[5 * G::Pos + e]);
     pl[e] = u;
     pl[G::OffV + e] = v;
+    const double huv = hu * w2;  // F_2 / 2 = G_1 / 2
     if (row >= 3 && row < 3 + TH) {
-      const double hu = 0.5 * u;
-#pragma unroll
-      for (int k = 0; k < 5; ++k)
-        pl[G::OffF + k * G::PF + (row - 3) * kBW64 + col] =
-            k == 1 ? fma(hu, tile[G::Pos + e], hp) : hu * tile[k * G::Pos + e];
+      double* f = pl + G::OffF + (row - 3) * kBW64 + col;
+      f[0] = half64(w1);
+      f[G::PF] = fma(hu, w1, hp);
+      f[2 * G::PF] = huv;
+      f[3 * G::PF] = hu * tile[3 * G::Pos + e];
+      f[4 * G::PF] = hu * tile[4 * G::Pos + e];
     }
     if (col >= 3 && col < 3 + 32) {
-      const double hv = 0.5 * v;
-#pragma unroll
-      for (int k = 0; k < 5; ++k)
-        pl[G::OffG + k * G::PG + row * 32 + (col - 3)] =
-            k == 2 ? fma(hv, tile[2 * G::Pos + e], hp) : hv * tile[k * G::Pos + e];
+      double* g = pl + G::OffG + row * 32 + (col - 3);
+      g[0] = half64(w2);
+      g[G::PG] = huv;
+      g[2 * G::PG] = fma(hv, w2, hp);
+      g[3 * G::PG] = hv * tile[3 * G::Pos + e];
+      g[4 * G::PG] = hv * tile[4 * G::Pos + e];
     }
   }
 }
@@ -112,74 +126,58 @@ __device__ __forceinline__ int switch64(const SAcc64P<TH>& A, const RhsConst& P)
 }
 
 // Viscous, entropy-production and relaxation sources H1..H4
-// (rhs_hybrid_high_llf.m4:161-237) from the planes.
+// (rhs_hybrid_high_llf.m4:161-237) from the planes, 72 FP64 operations.
+//
+// The reference's H3 = sigma - rho / T_n c_vn M_n + cond holds three pairs
+// that cancel: kappa |grad T|^2 / T^2 enters sigma with a plus and the
+// conduction with a minus, and with A_n = (T / T_n - 1) c_vn
+//   rho / T A_n M_n - rho / T_n c_vn M_n = -rho c_vn M_n / T.
+// What remains is (viscous heating + kappa lap T - c_vn H4) / T with H4 = rho
+// M_n.  The differences stay unscaled and the viscosities, the grid spacings
+// and the literals 4/3 and 2/3 are in the launch constants (visc_const); the
+// heating muB (u_x + v_y)^2 + mu/2 (phi_xx^2 + 2 phi_xy^2 + phi_yy^2) is the
+// quadratic form qa (u_x^2 + v_y^2) + qb u_x v_y + mu phi_xy^2.  As the
+// reference writes it the sources took 122 operations.
 template <int TH>
 __device__ __forceinline__ void sources64(const SAcc64P<TH>& A, const RhsConst& P, double H[5]) {
-  const double c43 = Lit::c4_3, c23 = Lit::c2_3;
-  double u[3][3], v[3][3];
-#pragma unroll
-  for (int dj = -1; dj <= 1; ++dj)
-#pragma unroll
-    for (int di = -1; di <= 1; ++di) {
-      u[dj + 1][di + 1] = A.u(di, dj);
-      v[dj + 1][di + 1] = A.v(di, dj);
-    }
-  double u_dxx = ((u[1][0] - 2.0 * u[1][1]) + u[1][2]) * P.inv_dx0sq;
-  double u_dyy = ((u[0][1] - 2.0 * u[1][1]) + u[2][1]) * P.inv_dx1sq;
-  double v_dxy = (((v[2][2] - v[0][2]) - v[2][0]) + v[0][0]) * P.inv_4dxdy;
-  H[1] = P.muB * (u_dxx + v_dxy) + P.mu * ((c43 * u_dxx - c23 * v_dxy) + (u_dyy + v_dxy));
-  double v_dyy = ((v[0][1] - 2.0 * v[1][1]) + v[2][1]) * P.inv_dx1sq;
-  double v_dxx = ((v[1][0] - 2.0 * v[1][1]) + v[1][2]) * P.inv_dx0sq;
-  double u_dyx = (((u[2][2] - u[0][2]) - u[2][0]) + u[0][0]) * P.inv_4dxdy;
-  H[2] = P.muB * (v_dyy + u_dyx) + P.mu * ((u_dyx + v_dxx) + (c43 * v_dyy - c23 * u_dyx));
-
-  double ux = (u[1][2] - u[1][0]) * P.inv_2dx0;
-  double uy = (u[2][1] - u[0][1]) * P.inv_2dx1;
-  double vy = (v[2][1] - v[0][1]) * P.inv_2dx1;
-  double vx = (v[1][2] - v[1][0]) * P.inv_2dx0;
-  const double Tc = A.t_(0, 0), txm = A.t_(-1, 0), txp = A.t_(1, 0), tym = A.t_(0, -1), typ = A.t_(0, 1);
-  double tx = (txp - txm) * P.inv_2dx0;
-  double ty = (typ - tym) * P.inv_2dx1;
-  double txx = ((txm - 2.0 * Tc) + txp) * P.inv_dx0sq;
-  double tyy = ((tym - 2.0 * Tc) + typ) * P.inv_dx1sq;
+  const double u0 = A.u(0, 0), v0 = A.v(0, 0);
+  const double ue = A.u(1, 0), uw = A.u(-1, 0), un = A.u(0, 1), us = A.u(0, -1);
+  const double ve = A.v(1, 0), vw = A.v(-1, 0), vn = A.v(0, 1), vs = A.v(0, -1);
+  {
+    const double uxx = fma(-2.0, u0, uw + ue), uyy = fma(-2.0, u0, us + un);
+    const double vxy = (A.v(1, 1) - A.v(1, -1)) - (A.v(-1, 1) - A.v(-1, -1));
+    H[1] = fma(P.h_long0, uxx, fma(P.h_mixed, vxy, P.h_trans1 * uyy));
+    const double vxx = fma(-2.0, v0, vw + ve), vyy = fma(-2.0, v0, vs + vn);
+    const double uxy = (A.u(1, 1) - A.u(1, -1)) - (A.u(-1, 1) - A.u(-1, -1));
+    H[2] = fma(P.h_long1, vyy, fma(P.h_mixed, uxy, P.h_trans0 * vxx));
+  }
+  const double Tc = A.t_(0, 0);
   const double rho = A.w(0, 0, 0);
-  double T_n = A.w(4, 0, 0) * rcp64(rho);
-  double Mn = (Tc - T_n) * P.inv_tau_n;
-  double inv_Tn = rcp64(T_n);
-  double tmp1 = P.T_star_n * inv_Tn;
-  double c_vn = ((Lit::c0_78 * P.R) * (tmp1 * tmp1)) * (fabs(tmp1) < 700.0 ? exp64(-tmp1) : exp(-tmp1));
-  double A_n = (Tc * inv_Tn - 1.0) * c_vn;
-  double phi_xx = c43 * ux - c23 * vy;
-  double phi_xy = uy + vx;
-  double phi_yy = c43 * vy - c23 * ux;
-  double inv_T = rcp64(Tc);
-  double inv_T2 = inv_T * inv_T;
-  double s0 = ux + vy;
-  double sigma = (((P.muB * inv_T) * (s0 * s0) +
-                   (P.mu * 0.5 * inv_T) * ((phi_xx * phi_xx + 2.0 * (phi_xy * phi_xy)) + phi_yy * phi_yy)) +
-                  (P.kappa * inv_T2) * (tx * tx + ty * ty)) +
-                 (rho * inv_T) * (A_n * Mn);
-  double cond = ((-(P.kappa * (tx * tx)) * inv_T2 + (P.kappa * txx) * inv_T) - (P.kappa * (ty * ty)) * inv_T2) +
-                (P.kappa * tyy) * inv_T;
-  H[3] = (sigma - ((rho * inv_Tn) * c_vn) * Mn) + cond;
+  const double T_n = A.w(4, 0, 0) * rcp64(rho);
   H[4] = (rho * P.inv_tau_n) * (Tc - T_n);
+  const double tmp1 = P.T_star_n * rcp64(T_n);
+  const double c_vn = (P.R078 * (tmp1 * tmp1)) * (fabs(tmp1) < 700.0 ? exp64(-tmp1) : exp(-tmp1));
+  const double ux = (ue - uw) * P.inv_2dx0, vy = (vn - vs) * P.inv_2dx1;
+  const double phi = fma(un - us, P.inv_2dx1, (ve - vw) * P.inv_2dx0);
+  const double heat = fma(ux, fma(P.q_b, vy, P.q_a * ux), fma(P.q_a * vy, vy, (P.mu * phi) * phi));
+  const double txx = fma(-2.0, Tc, A.t_(-1, 0) + A.t_(1, 0)), tyy = fma(-2.0, Tc, A.t_(0, -1) + A.t_(0, 1));
+  H[3] = rcp64(Tc) * fma(-c_vn, H[4], fma(P.k_0, txx, fma(P.k_1, tyy, heat)));
 }
 
-// Flux part of the five fields of a DRP cell, dF/dx + dG/dy (Tam-Webb,
-// rhs_hybrid_high_llf.m4:258-268).  The planes hold half fluxes: the
-// coefficients are doubled (exactly).
+// K = H - dF/dx - dG/dy of the five fields of a DRP cell (Tam-Webb,
+// rhs_hybrid_high_llf.m4:258-268), H overwritten.  The coefficients are divided
+// by the first one, which the launch constants drp_0 and drp_1 hold with the
+// grid spacing and a factor 2 for the planes' half fluxes.
 template <int TH>
-__device__ __forceinline__ void drp_flux64(const SAcc64P<TH>& A, const RhsConst& P, double D[5]) {
+__device__ __forceinline__ void drp_flux64(const SAcc64P<TH>& A, const RhsConst& P, double H[5]) {
+  constexpr double b2 = Lit::a2 / Lit::a1, b3 = Lit::a3 / Lit::a1;
 #pragma unroll
   for (int k = 0; k < 5; ++k) {
-    double fx = 0.0, gy = 0.0;
-#pragma unroll
-    for (int m = 3; m >= 1; --m) {
-      const double a = 2.0 * (m == 1 ? Lit::a1 : (m == 2 ? Lit::a2 : Lit::a3));
-      fx = fma(a, A.fx(k, m) - A.fx(k, -m), fx);
-      gy = fma(a, A.gy(k, m) - A.gy(k, -m), gy);
-    }
-    D[k] = fma(fx, P.inv_dx0, gy * P.inv_dx1);
+    const double fx =
+        fma(b3, A.fx(k, 3) - A.fx(k, -3), fma(b2, A.fx(k, 2) - A.fx(k, -2), A.fx(k, 1) - A.fx(k, -1)));
+    const double gy =
+        fma(b3, A.gy(k, 3) - A.gy(k, -3), fma(b2, A.gy(k, 2) - A.gy(k, -2), A.gy(k, 1) - A.gy(k, -1)));
+    H[k] = fma(-fx, P.drp_0, fma(-gy, P.drp_1, H[k]));
   }
 }
 
@@ -273,11 +271,11 @@ __device__ __forceinline__ void weno_tasks64(const double* tile, const double* p
     D[part * (32 * TH) + cell] = c * d;
   }
 }
-// dF/dx + dG/dy of field k of a WENO cell from weno_tasks64's parts.
+// -(dF/dx + dG/dy) of field k of a WENO cell from weno_tasks64's parts.
 template <int TH>
 __device__ __forceinline__ double weno_part64(const double* D, int cell, int k) {
-  if constexpr (kFluxParts64<TH> == 5) return -D[k * (32 * TH) + cell];
-  else return -(D[k * (32 * TH) + cell] + D[(k + 5) * (32 * TH) + cell]);
+  if constexpr (kFluxParts64<TH> == 5) return D[k * (32 * TH) + cell];
+  else return D[k * (32 * TH) + cell] + D[(k + 5) * (32 * TH) + cell];
 }
 
 // Accessor of the learned switch's features on an FP64 tile: density and

@@ -88,17 +88,17 @@ __global__ void __launch_bounds__(256, 2)
   if (!valid) return;
   const SAcc64P<TH> A = acc64p<TH>(tile, pl, lane, warp);
   const long o = (long)(j0 + warp) * opitch + (i0 + lane);
-  double H[5], D[5];
+  double H[5];
   H[0] = H0[o];
   sources64(A, P, H);
   if (flag) {
 #pragma unroll
-    for (int k = 0; k < 5; ++k) D[k] = weno_part64<TH>(flux, tid, k);
+    for (int k = 0; k < 5; ++k) H[k] += weno_part64<TH>(flux, tid, k);
   } else {
-    drp_flux64(A, P, D);
+    drp_flux64(A, P, H);
   }
 #pragma unroll
-  for (int k = 0; k < 5; ++k) KK[k * ofstride + o] = H[k] - D[k];
+  for (int k = 0; k < 5; ++k) KK[k * ofstride + o] = H[k];
   if (flags) flags[o] = flag;
 }
 
@@ -389,6 +389,19 @@ RhsConst make_rhs_const(const double* xlo, const double* dx, double alpha, doubl
   P.sensor_eps = ((Lit::c0_9 * tol[2]) * (xi * xi)) / (1.0 - Lit::c0_9 * (tol[2] * tol[2]));
   P.sensor_eps32 = ratio_eps32(P.sensor_eps);
   P.level = level;
+  const double lon = muB + Lit::c4_3 * mu, mix = muB + (1.0 - Lit::c2_3) * mu;
+  P.h_long0 = lon * P.inv_dx0sq;
+  P.h_long1 = lon * P.inv_dx1sq;
+  P.h_trans0 = mu * P.inv_dx0sq;
+  P.h_trans1 = mu * P.inv_dx1sq;
+  P.h_mixed = mix * P.inv_4dxdy;
+  P.q_a = muB + 0.5 * mu * (Lit::c4_3 * Lit::c4_3 + Lit::c2_3 * Lit::c2_3);
+  P.q_b = 2.0 * muB - 2.0 * mu * (Lit::c4_3 * Lit::c2_3);
+  P.k_0 = kappa * P.inv_dx0sq;
+  P.k_1 = kappa * P.inv_dx1sq;
+  P.R078 = Lit::c0_78 * R;
+  P.drp_0 = 2.0 * Lit::a1 * P.inv_dx0;
+  P.drp_1 = 2.0 * Lit::a1 * P.inv_dx1;
   return P;
 }
 

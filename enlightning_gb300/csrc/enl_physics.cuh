@@ -29,6 +29,11 @@ struct RhsConst {
   double ylo, dy;                   // height of row j: ylo + dy*((j - jfirst) + 0.5)
   double sensor_eps;                // ep of the hybrid sensor (tolerance(2))
   float sensor_eps32;               // ratio_eps32 of it
+  // FP64 sources and DRP differences (enl_cell64.cuh): coefficients of the
+  // unscaled second differences in H1 and H2 (along a component's own
+  // direction 0 or 1, across it, mixed), of the heating's quadratic form, of
+  // the unscaled Laplacian of T, 0.78 R, and 2 a1 / dx
+  double h_long0, h_long1, h_trans0, h_trans1, h_mixed, q_a, q_b, k_0, k_1, R078, drp_0, drp_1;
   int level;
 };
 
