@@ -1003,7 +1003,10 @@ __global__ void __launch_bounds__(256, std::is_same<S, float>::value ? kStageBlo
           __syncthreads();
         }
         weno_tasks64<ORDER, LLF, kTH>(tile, planes64, A.P[lvl], j0, w, h, all ? nullptr : s_list, nw, flux64);
-        __syncthreads();
+        // a full tile's warp w has done row w's tasks, and its lanes read back
+        // what they wrote themselves: no barrier, so that the warps' FP64 and
+        // FP32 phases drift apart
+        if (!(all && h == kTH)) __syncthreads();
       }
       if (direct ? valid : (tid < nd + nw)) {
         const int e = direct ? ((ty << 5) | tx | (FAST ? (SCHEME == kWeno ? 1 << 16 : 0) : flag << 16)) : s_list[tid];
