@@ -403,76 +403,89 @@ __device__ __forceinline__ S uni_key(const S* box, const S* first, int un_is_in,
   return k < 7 ? box[k * kPl] : (k < 12 ? (un_is_in ? box[(k - 7) * kPl] : first[k - 7]) : first[5]);
 }
 
-// The uniform-tile test of the stage kernel, in two out-of-line parts (the
-// stage kernel's cell computation keeps its registers) around one block
-// barrier in the kernel.  uniform_probe: this thread's part of the test, after
-// the tile's halo box has landed in `box` (kPl elements per field, rows of
-// kRow): its share of the box equals each field's first element, and its
-// cell's u^n and H0 equal those of the first cell of its warp, whose values
-// lane 0 writes to wl[warp] (the caller loaded them before the tile's wait,
-// zero in stage 1 where u^n is the staged box).  uniform_hit, after the barrier's AND of the
-// probes: 0 when the tile is not uniform; 1 when it is and the level's cache
-// entry holds its inputs (the cached outputs are stored into every cell of
-// the tile and counted); 2 when it is uniform and must be computed (the
-// caller's cell (0, 0) then fills the entry).  Neither contains a barrier.
+// The uniform-tile test of the stage kernel, after the tile's halo box has
+// landed in `box` (kPl elements per field, rows of kRow).
+//
+// uniform_maybe: 32 samples of the box (8 positions of rho, rho u, rho v and
+// rho T_n, one per lane) against each field's first element.  Every warp takes
+// the same samples, so the answer is the block's without a barrier; a tile
+// that a wave has reached fails here, and the full test costs what it costs
+// for tiles that pass.  (Testing every tile's box in full, with the cells'
+// u^n and H0 exchanged through shuffles and shared memory, was a third of the
+// cycles of an FP32-storage tile that is not uniform: 5,000-7,000 of 17,000.)
 template <typename S, int kPl, int kRow>
-__device__ __noinline__ bool uniform_probe(const S* box, S (*wl)[6], int w, int h, S u0, S u1, S u2, S u3, S u4,
-                                           S hv) {
+__device__ __forceinline__ bool uniform_maybe(const S* box) {
+  const int lane = threadIdx.x & 31, q = lane >> 2;
+  const int k = (lane & 3) == 3 ? 4 : (lane & 3);
+  // positions over the 38 x 14 box: its far corners, edges and middle
+  const int col = (q & 1) ? 37 - 5 * (q >> 1) : 12 * (q >> 1), row = (q & 2) ? 13 - (q & 1) - (q >> 2) : 3 * (q >> 2) + 4 * (q & 1);
+  return __all_sync(0xffffffffu, same_bits(box[k * kPl + row * kRow + col], box[k * kPl]));
+}
+
+// The full test, in two out-of-line parts (the stage kernel's cell computation
+// keeps its registers) around one block barrier in the kernel.  uniform_probe:
+// this thread's part: warp k < 7 holds field k of the box against its first
+// element, 16 bytes at a time, and every cell's u^n and H0 must equal those of
+// the tile's first cell (both loaded before the tile's wait; zero in stage 1
+// for u^n, which is the staged box).  uniform_hit, after the barrier's AND of
+// the probes: 1 when the level's cache entry holds the tile's inputs (the
+// cached outputs are stored into every cell of the tile and counted); 2 when
+// the tile must be computed (the caller's cell (0, 0) then fills the entry).
+// Neither contains a barrier; `first` (u^n and H0 of the first cell) is shared.
+template <typename S, int kPl, int kRow>
+__device__ __noinline__ bool uniform_probe(const S* box, S* first, int w, int h, S u0, S u1, S u2, S u3, S u4, S hv,
+                                           S f0, S f1, S f2, S f3, S f4, S fh) {
   const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
-  const bool valid = lane < w && warp < h;
-  const S v[6] = {u0, u1, u2, u3, u4, hv};  // u^n (5 fields) and H0 of this thread's cell
-  // the staged box 16 bytes at a time, every element against its field's
-  // first element (bit patterns OR-ed together: zero when all equal)
-  bool ok;
-  if constexpr (std::is_same<S, double>::value) {
-    static_assert(kRow == 38 && kPl == 532, "FP64 box: rows of 38, 14 rows");
-    const double2* b2 = reinterpret_cast<const double2*>(box);
-    unsigned long long acc = 0ull;
-    for (int q = tid; q < kNF * (kPl / 2); q += 256) {
-      const int k = q / (kPl / 2);
-      const unsigned long long ref = (unsigned long long)__double_as_longlong(box[k * kPl]);
-      const double2 x = b2[q];
-      acc |= ((unsigned long long)__double_as_longlong(x.x) ^ ref) | ((unsigned long long)__double_as_longlong(x.y) ^ ref);
+  bool ok = true;
+  if (warp < kNF) {
+    const S* p = box + warp * kPl;
+    if constexpr (std::is_same<S, double>::value) {
+      static_assert(kRow == 38 && kPl == 532, "FP64 box: rows of 38, 14 rows");
+      const unsigned long long ref = (unsigned long long)__double_as_longlong(p[0]);
+      const double2* b2 = reinterpret_cast<const double2*>(p);
+      unsigned long long acc = 0ull;
+      for (int q = lane; q < kPl / 2; q += 32) {
+        const double2 x = b2[q];
+        acc |= ((unsigned long long)__double_as_longlong(x.x) ^ ref) | ((unsigned long long)__double_as_longlong(x.y) ^ ref);
+      }
+      ok = acc == 0ull;
+    } else {
+      static_assert(kRow == 40 && kPl == 560, "FP32 box: rows of 40 (38 used), 14 rows");
+      const unsigned ref = __float_as_uint(p[0]);
+      const float4* b4 = reinterpret_cast<const float4*>(p);
+      unsigned acc = 0u;
+      int cv = lane % 10;  // 16-byte column of the row; columns 38, 39 are unused
+      for (int q = lane; q < kPl / 4; q += 32) {
+        const float4 x = b4[q];
+        acc |= (__float_as_uint(x.x) ^ ref) | (__float_as_uint(x.y) ^ ref);
+        if (cv != 9) acc |= (__float_as_uint(x.z) ^ ref) | (__float_as_uint(x.w) ^ ref);
+        cv = cv >= 8 ? cv - 8 : cv + 2;  // 32 = 2 mod 10
+      }
+      ok = acc == 0u;
     }
-    ok = acc == 0ull;
-  } else {
-    static_assert(kRow == 40 && kPl == 560, "FP32 box: rows of 40 (38 used), 14 rows");
-    const float4* b4 = reinterpret_cast<const float4*>(box);
-    unsigned acc = 0u;
-    for (int q = tid; q < kNF * (kPl / 4); q += 256) {
-      const int k = q / (kPl / 4), cv = (q - k * (kPl / 4)) % (kRow / 4);
-      const unsigned ref = __float_as_uint(box[k * kPl]);
-      const float4 x = b4[q];
-      unsigned d = (__float_as_uint(x.x) ^ ref) | (__float_as_uint(x.y) ^ ref);
-      if (cv != kRow / 4 - 1) d |= (__float_as_uint(x.z) ^ ref) | (__float_as_uint(x.w) ^ ref);  // columns 38, 39 unused
-      acc |= d;
-    }
-    ok = acc == 0u;
   }
-  // every lane takes part in the shuffle (a lane without a cell included:
-  // the full-mask shuffle waits for all 32), only cells compare
-#pragma unroll
-  for (int k = 0; k < 6; ++k) {
-    const S first = __shfl_sync(0xffffffffu, v[k], 0);
-    if (valid && !same_bits(v[k], first)) ok = false;
-    if (lane == 0 && valid) wl[warp][k] = v[k];
+  if (lane < w && warp < h)
+    ok = ok && same_bits(u0, f0) && same_bits(u1, f1) && same_bits(u2, f2) && same_bits(u3, f3) && same_bits(u4, f4) &&
+         same_bits(hv, fh);
+  if (tid == 0) {
+    first[0] = f0;
+    first[1] = f1;
+    first[2] = f2;
+    first[3] = f3;
+    first[4] = f4;
+    first[5] = fh;
   }
   return ok;
 }
 
 template <typename S, int kPl>
-__device__ __noinline__ int uniform_hit(const StageArgs& A, const S* box, const UniEntry<S>* uc, const S (*wl)[6],
+__device__ __noinline__ int uniform_hit(const StageArgs& A, const S* box, const UniEntry<S>* uc, const S* first,
                                         unsigned* stats, int lvl, int i0, int j0, int w, int h) {
-  for (int q = 1; q < h; ++q)
-#pragma unroll
-    for (int k = 0; k < 6; ++k)
-      if (!same_bits(wl[q][k], wl[0][k])) return 0;
-  const UniEntry<S>& U = uc[lvl];
-  bool hit = U.valid != 0;
-#pragma unroll
-  for (int k = 0; k < 13; ++k) hit = hit && same_bits(uni_key<S, kPl>(box, wl[0], A.un_is_in, k), U.key[k]);
-  if (!hit) return 2;
   const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+  const UniEntry<S>& U = uc[lvl];
+  const bool hit = __all_sync(0xffffffffu, U.valid != 0 && (lane >= 13 || same_bits(uni_key<S, kPl>(box, first, A.un_is_in, lane),
+                                                                                   U.key[lane])));
+  if (!hit) return 2;
   if (lane < w && warp < h) {
     S* out = static_cast<S*>(A.out[lvl]);
     const long fs = A.fstride[lvl];
@@ -654,7 +667,7 @@ __global__ void __launch_bounds__(256, std::is_same<S, float>::value ? kStageBlo
   __shared__ int s_list[256];
   __shared__ TileInfo s_tile;
   __shared__ UniEntry<S> s_uc[kL];
-  __shared__ S s_wl[8][6];  // per warp: u^n (5 fields) and H0 of its first cell
+  __shared__ S s_first[6];  // u^n (5 fields) and H0 of the tile's first cell (uniform tiles)
   const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
   const int ntiles = *A.ntiles;
   const int tbase = A.tile_base ? *A.tile_base : 0;
@@ -752,15 +765,22 @@ __global__ void __launch_bounds__(256, std::is_same<S, float>::value ? kStageBlo
     const int i0 = td.x, j0 = td.y;
     const int tx = lane, ty = warp;
     const bool valid = tx < w && ty < h;
-    // u^n and H0 of this thread's cell, for the uniform-tile test: loaded
-    // before the wait, so that their latency overlaps it
+    // u^n and H0 of this thread's cell and of the tile's first cell, for the
+    // uniform-tile test: loaded before the wait, so that their latency
+    // overlaps it
     S un_c[5] = {S(0), S(0), S(0), S(0), S(0)}, h0_c = S(0);
-    if (A.uniform && valid) {
-      const long g = (long)(j0 + ty + 3) * A.pitch[lvl] + (i0 + tx + 3);
+    S un_f[5] = {S(0), S(0), S(0), S(0), S(0)}, h0_f = S(0);
+    if (A.uniform) {
+      const long g0 = (long)(j0 + 3) * A.pitch[lvl] + (i0 + 3);
+      const long g = valid ? g0 + (long)ty * A.pitch[lvl] + tx : g0;
       h0_c = static_cast<const S*>(A.h0[lvl])[g];
+      h0_f = static_cast<const S*>(A.h0[lvl])[g0];
       if (!A.un_is_in)
 #pragma unroll
-        for (int k = 0; k < 5; ++k) un_c[k] = static_cast<const S*>(A.un[lvl])[k * A.fstride[lvl] + g];
+        for (int k = 0; k < 5; ++k) {
+          un_c[k] = static_cast<const S*>(A.un[lvl])[k * A.fstride[lvl] + g];
+          un_f[k] = static_cast<const S*>(A.un[lvl])[k * A.fstride[lvl] + g0];
+        }
     }
 #if ENL_PREFETCH_UN
     if constexpr (kF32S && !kUnTma) {
@@ -799,17 +819,20 @@ __global__ void __launch_bounds__(256, std::is_same<S, float>::value ? kStageBlo
     int ucode = 0;
     if (A.uniform) {
       const S* box = reinterpret_cast<const S*>(dst[b]);
-      const bool ok = uniform_probe<S, kPl, kF32S ? kBW32 : kBW>(box, s_wl, w, h, un_c[0], un_c[1], un_c[2],
-                                                                 un_c[3], un_c[4], h0_c);
-      const bool all = __syncthreads_and(ok) != 0;  // (also publishes s_tile and s_wl)
-      if (all && s_tile.absorb == 0) ucode = uniform_hit<S, kPl>(A, box, s_uc, s_wl, s_stats, lvl, i0, j0, w, h);
+      if (uniform_maybe<S, kPl, kF32S ? kBW32 : kBW>(box)) {
+        const bool ok = uniform_probe<S, kPl, kF32S ? kBW32 : kBW>(box, s_first, w, h, un_c[0], un_c[1], un_c[2],
+                                                                   un_c[3], un_c[4], h0_c, un_f[0], un_f[1], un_f[2],
+                                                                   un_f[3], un_f[4], h0_f);
+        const bool all = __syncthreads_and(ok) != 0;  // (also publishes s_tile and s_first)
+        if (all && s_tile.absorb == 0) ucode = uniform_hit<S, kPl>(A, box, s_uc, s_first, s_stats, lvl, i0, j0, w, h);
+      }
       // this step's records of the tile (a computed uniform tile, ucode 2,
       // records its outputs where its first cell records the cache entry)
       if (tid == 0 && A.rec_un_out) {
         UnRec<S>* rn = static_cast<UnRec<S>*>(A.rec_un_out) + gti;
         if (ucode != 0)
 #pragma unroll
-          for (int k = 0; k < 6; ++k) rn->v[k] = uni_key<S, kPl>(box, s_wl[0], A.un_is_in, 7 + k);
+          for (int k = 0; k < 6; ++k) rn->v[k] = uni_key<S, kPl>(box, s_first, A.un_is_in, 7 + k);
         rn->valid = ucode != 0 ? 1 : 0;
       }
       if (tid == 0 && A.rec_out && ucode != 2) {
@@ -1060,7 +1083,7 @@ __global__ void __launch_bounds__(256, std::is_same<S, float>::value ? kStageBlo
           out[5 * fs + g] = pq;
           out[6 * fs + g] = tp;
           if (record) {
-            uniform_record<S, kPl>(&s_uc[lvl], reinterpret_cast<const S*>(dst[b]), s_wl[0], A.un_is_in, wn[0], wn[1],
+            uniform_record<S, kPl>(&s_uc[lvl], reinterpret_cast<const S*>(dst[b]), s_first, A.un_is_in, wn[0], wn[1],
                                    wn[2], wn[3], wn[4], pq, tp, f);
             if (A.rec_out) record_out<S>(static_cast<OutRec<S>*>(A.rec_out) + gti, wn, pq, tp);
             if (A.gcache) publish_uniform<S>(static_cast<GUni<S>*>(A.gcache) + lvl, s_uc[lvl]);
@@ -1137,7 +1160,7 @@ __global__ void __launch_bounds__(256, std::is_same<S, float>::value ? kStageBlo
 #pragma unroll
           for (int k = 0; k < 5; ++k) out[k * fs + g] = wn[k];
           if (record) {
-            uniform_record<S, kPl>(&s_uc[lvl], reinterpret_cast<const S*>(dst[b]), s_wl[0], A.un_is_in, wn[0], wn[1],
+            uniform_record<S, kPl>(&s_uc[lvl], reinterpret_cast<const S*>(dst[b]), s_first, A.un_is_in, wn[0], wn[1],
                                    wn[2], wn[3], wn[4], pv, tv, f);
             if (A.rec_out) record_out<S>(static_cast<OutRec<S>*>(A.rec_out) + gti, wn, pv, tv);
             if (A.gcache) publish_uniform<S>(static_cast<GUni<S>*>(A.gcache) + lvl, s_uc[lvl]);
