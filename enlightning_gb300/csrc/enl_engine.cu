@@ -153,13 +153,14 @@ __device__ __forceinline__ int absorb_reach(const AbsorbTables& T, int lvl, int 
 }
 
 // Sides whose walk can reach some cell of the w x h tile at (i0, j0) of patch
-// b with a factor other than exactly 1: the continuation tests are monotone,
+// b with a factor other than exactly 1 (host, over the host's copy of the
+// tables; the tile table carries it in bits 24..27 of a descriptor's .z): the continuation tests are monotone,
 // so the tile's cell nearest to each side decides.  (The walk from a patch's
 // own edge reaches its first cell even far from the domain side, where the
 // factor is exactly 1; the batched engine leaves such cells as they are,
 // which is the reference's (q - q_amb) * 1 + q_amb except for a last-place
 // rounding when q is beyond twice its ambient value.)
-__device__ __forceinline__ int absorb_tile_mask(const AbsorbTables& T, int lvl, int i0, int j0, int w, int h,
+inline int absorb_tile_mask(const AbsorbTables& T, int lvl, int i0, int j0, int w, int h,
                                                 const int4& b) {
   int m = 0;
   const unsigned char* c = T.cont[lvl][0];
@@ -172,14 +173,6 @@ __device__ __forceinline__ int absorb_tile_mask(const AbsorbTables& T, int lvl, 
   if (c && j0 + h - 1 >= T.act[lvl][3] && c[b.w] && (j0 + h - 1 == b.w || c[j0 + h])) m |= 8;
   return m;
 }
-
-// Per-tile values computed once by thread 0 and read by every thread after
-// the next barrier.
-struct TileInfo {
-  int4 box;       // the tile's patch
-  int absorb;     // absorb_tile_mask
-  float bdtf;     // beta * dt in single precision
-};
 
 // (q - ambient) * tmp + ambient, rounding like the reference's statement
 __device__ __forceinline__ double relax_(double q, double amb, double tmp) {
@@ -493,7 +486,7 @@ __device__ __noinline__ int uniform_hit(const StageArgs& A, const S* box, const 
 #pragma unroll
     for (int k = 0; k < kNF; ++k) out[k * fs + gc] = U.res[k];
   }
-  if (tid == 0) {
+  if (tid == 64) {  // (thread 0 stages the next tile, thread 32 writes the records)
     stats[4 * lvl + 0] += U.weno ? (unsigned)(w * h) : 0u;
     stats[4 * lvl + 1] += (unsigned)(w * h);
     stats[4 * lvl + 3] += (unsigned)(w * h);
@@ -665,16 +658,24 @@ __global__ void __launch_bounds__(256, std::is_same<S, float>::value ? kStageBlo
   __shared__ unsigned s_stats[4 * kL];
   __shared__ int s_cnt[2][8];
   __shared__ int s_list[256];
-  __shared__ TileInfo s_tile;
+  __shared__ __align__(16) int4 s_dq;  // descriptor and table index on their way (thread 0)
+  __shared__ int s_gq;
+  __shared__ int s_run;  // end of the block's run of claimed tiles (thread 0)
   __shared__ UniEntry<S> s_uc[kL];
   __shared__ S s_first[6];  // u^n (5 fields) and H0 of the tile's first cell (uniform tiles)
   const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
   const int ntiles = *A.ntiles;
   const int tbase = A.tile_base ? *A.tile_base : 0;
-  // the block's next tile: the rest of its run of A.chunk consecutive tiles
-  // (neighbours in the table: the next tile to the right in a patch row),
-  // then a new run from the counter
-  auto claim_next = [&](int cur) -> int {
+  // Claims (thread 0).  A block takes a run of consecutive tiles per claim:
+  // A.chunk of them (neighbours in the table: the next tile to the right in a
+  // patch row) or, with A.chunk = 1, an eighth of its share of what is left, at
+  // most 8 and down to single tiles towards the end, where they balance the
+  // blocks.  Inside a run the next tile is known, so its descriptor is on its
+  // way while the current tile is worked on; thread 0 sits out the counter's
+  // and the descriptor's global latency (with single claims 3,900 of the
+  // 14,000 cycles of a uniform tile, the block waiting at its next barrier)
+  // once per run.
+  auto claim = [&](int cur) -> int {
     if (A.tile_order == 3) {
       // two streams on one packed counter (level-0 claims in the low half,
       // finest-end claims in the high half): the first wave of blocks (one
@@ -689,20 +690,31 @@ __global__ void __launch_bounds__(256, std::is_same<S, float>::value ? kStageBlo
       if (f + bk >= (unsigned long long)ntiles) return ntiles;
       return from_end ? ntiles - 1 - (int)bk : (int)f;
     }
-    if (cur >= 0 && (cur + 1) % A.chunk != 0 && cur + 1 < ntiles) return cur + 1;
-    return atomicAdd(A.counter, A.chunk);
+    if (cur + 1 < s_run) return cur + 1;
+    const int n = A.chunk > 1 ? A.chunk : min(8, max(1, (ntiles - s_run) / (8 * (int)gridDim.x)));
+    const int t = atomicAdd(A.counter, n);
+    s_run = t + n;
+    return t;
   };
-  auto issue = [&](int t, int b) {
+  auto fetch = [&](int t) {
+    if (t >= ntiles) return;
     // claim order -> table index (the table runs level 0 to the finest);
     // order 2 takes the two ends alternately, so that fine-level WENO tiles
     // (FP64-bound) and level-0 tiles (memory-bound) run side by side
     const int ti = (A.tile_order == 1 || A.tile_order == 3) ? t  // order 3 claims table indices
                    : A.tile_order == 2 ? ((t & 1) ? (t >> 1) : ntiles - 1 - (t >> 1))
                                        : ntiles - 1 - t;
-    const int4 td = A.tiles[tbase + ti];
-    const int gi = A.gti ? A.gti[tbase + ti] : tbase + ti;
+    cp_async<16>(&s_dq, A.tiles + tbase + ti);
+    if (A.gti) cp_async<4>(&s_gq, A.gti + tbase + ti);
+    else s_gq = tbase + ti;
+  };
+  auto issue = [&](int t, int b) {
+    cp_async_wait();
+    const int4 td = s_dq;
+    const int gi = s_gq;
     s_td[b] = td;
     s_ti[b] = gi;
+    if (t + 1 < s_run) fetch(t + 1);  // (s_dq has been read)
     // a tiled TMA copy needs x * sizeof(S) to be a multiple of 16: x even for
     // doubles, a multiple of 4 for floats; set_patches only accepts such
     // patch origins and tiles are 32 wide
@@ -743,17 +755,22 @@ __global__ void __launch_bounds__(256, std::is_same<S, float>::value ? kStageBlo
     mbar_init(&mbar[0], 1);
     mbar_init(&mbar[1], 1);
     fence_mbar_init();
-    int t = claim_next(-1);
+    s_run = 0;
+    int t = claim(-1);
+    fetch(t);
     if (t < ntiles && !issue(t, 0)) t = ntiles;
     s_t[0] = t;
   }
   __syncthreads();
+  const float bdtf = kF32S ? (A.dtf_dev ? A.betaf * (*A.dtf_dev) : A.bdtf) : 0.f;
   uint32_t phase[2] = {0u, 0u};
   int b = 0;
   int t = s_t[0];
   while (t < ntiles) {
     if (tid == 0) {
-      int nt = claim_next(t);
+      const bool ahead = t + 1 < s_run;  // its descriptor is on its way
+      int nt = claim(t);
+      if (!ahead) fetch(nt);
       if (nt < ntiles && !issue(nt, b ^ 1)) nt = ntiles;
       s_t[b ^ 1] = nt;
     }
@@ -808,12 +825,7 @@ __global__ void __launch_bounds__(256, std::is_same<S, float>::value ? kStageBlo
     phase[b] ^= 1u;
     // beta*dt of this stage (dt from the device CFL reduction when adaptive)
     const double bdt = kF32S ? 0.0 : (A.dt_dev ? A.beta * (*A.dt_dev) : A.bdt);
-    if (tid == 0) {
-      const int4 pb = A.patchtab[td.w];
-      s_tile.box = pb;
-      s_tile.absorb = A.any_absorb ? absorb_tile_mask(A.absorb, lvl, i0, j0, w, h, pb) : 0;
-      s_tile.bdtf = A.dtf_dev ? A.betaf * (*A.dtf_dev) : A.bdtf;
-    }
+    const int absorb = (td.z >> 24) & 15;  // sides whose envelope reaches the tile
     // ---- uniform tile: one value per staged field, shared u^n and H0 ----
     constexpr int kPl = kF32S ? kPlane32 : kBH * kBW;  // elements per staged field
     int ucode = 0;
@@ -823,19 +835,20 @@ __global__ void __launch_bounds__(256, std::is_same<S, float>::value ? kStageBlo
         const bool ok = uniform_probe<S, kPl, kF32S ? kBW32 : kBW>(box, s_first, w, h, un_c[0], un_c[1], un_c[2],
                                                                    un_c[3], un_c[4], h0_c, un_f[0], un_f[1], un_f[2],
                                                                    un_f[3], un_f[4], h0_f);
-        const bool all = __syncthreads_and(ok) != 0;  // (also publishes s_tile and s_first)
-        if (all && s_tile.absorb == 0) ucode = uniform_hit<S, kPl>(A, box, s_uc, s_first, s_stats, lvl, i0, j0, w, h);
+        const bool all = __syncthreads_and(ok) != 0;  // (also publishes s_first)
+        if (all && absorb == 0) ucode = uniform_hit<S, kPl>(A, box, s_uc, s_first, s_stats, lvl, i0, j0, w, h);
       }
       // this step's records of the tile (a computed uniform tile, ucode 2,
       // records its outputs where its first cell records the cache entry)
-      if (tid == 0 && A.rec_un_out) {
+      // (thread 32: thread 0 has the next tile's staging on its hands)
+      if (tid == 32 && A.rec_un_out) {
         UnRec<S>* rn = static_cast<UnRec<S>*>(A.rec_un_out) + gti;
         if (ucode != 0)
 #pragma unroll
           for (int k = 0; k < 6; ++k) rn->v[k] = uni_key<S, kPl>(box, s_first, A.un_is_in, 7 + k);
         rn->valid = ucode != 0 ? 1 : 0;
       }
-      if (tid == 0 && A.rec_out && ucode != 2) {
+      if (tid == 32 && A.rec_out && ucode != 2) {
         OutRec<S>* ro = static_cast<OutRec<S>*>(A.rec_out) + gti;
         if (ucode == 1)
 #pragma unroll
@@ -1053,7 +1066,7 @@ __global__ void __launch_bounds__(256, std::is_same<S, float>::value ? kStageBlo
           H[0] = kUnTma ? h0b[ci] : static_cast<const float*>(A.h0[lvl])[g];
           sources_fast(acc, A.F[lvl], H);
           fluxes_fast<ORDER, LLF>(acc, A.F[lvl], gj, f, H, K);
-          const float a1 = A.a1f, a2 = A.a2f, bdtf = s_tile.bdtf;
+          const float a1 = A.a1f, a2 = A.a2f;
 #pragma unroll
           for (int k = 0; k < 5; ++k) {
             const float w = tile32[k * kPlane32 + c32];
@@ -1066,8 +1079,8 @@ __global__ void __launch_bounds__(256, std::is_same<S, float>::value ? kStageBlo
           const float rho = F.rho0 + wn[0];
           float pq, tp;
           eos_pert32(A.E32, wn[0], wn[3], row_height32(F.ylo, F.dy, gj), pq, tp);
-          if (s_tile.absorb) {  // perturbations relax towards 0
-            const int reach = absorb_reach(A.absorb, lvl, gi, gj, s_tile.box, s_tile.absorb);
+          if (absorb) {  // perturbations relax towards 0
+            const int reach = absorb_reach(A.absorb, lvl, gi, gj, A.patchtab[td.w], absorb);
 #pragma unroll
             for (int sd = 0; sd < 4; ++sd) {
               if (!(reach & (1 << sd))) continue;
@@ -1139,8 +1152,8 @@ __global__ void __launch_bounds__(256, std::is_same<S, float>::value ? kStageBlo
             // update_state (update_state.m4:90-105), as the state upload computes it
             eos64(A.E64, wn[0], wn[3], row_height64(A.ylo, A.dy[lvl], gj), pv, tv);
           }
-          if (s_tile.absorb) {  // absolute values relax towards the ambient state
-            const int reach = absorb_reach(A.absorb, lvl, gi, gj, s_tile.box, s_tile.absorb);
+          if (absorb) {  // absolute values relax towards the ambient state
+            const int reach = absorb_reach(A.absorb, lvl, gi, gj, A.patchtab[td.w], absorb);
             const double rT = __dmul_rn(A.T0, A.rho0);
 #pragma unroll
             for (int sd = 0; sd < 4; ++sd) {
@@ -2381,6 +2394,7 @@ struct Engine {
   cudaEvent_t stage_ev = nullptr;
   float* d_envf[kL][4] = {};
   unsigned char* d_cont[kL][4] = {};
+  std::vector<unsigned char> h_cont[kL][4];  // the host's copy
   double off[kNF] = {0, 0, 0, 0, 0, 0, 0};
 };
 
@@ -2606,6 +2620,10 @@ static long long band_cells(int nx, int ny, int sides) {
 // E->tables_from are unchanged since the last rebuild: their entries (at the
 // front of every table) are kept on the host and, unless a device table was
 // reallocated, on the device; only the rest is rebuilt and copied.
+static bool any_absorb(const Engine* E);
+static AbsorbTables absorb_tables(const Engine* E);
+static AbsorbTables absorb_tables_host(const Engine* E);
+
 static int rebuild_tables(Engine* E) {
   const int nl = E->cfg.nlevels;
   const int l0 = std::min(E->tables_from, nl);
@@ -2632,7 +2650,15 @@ static int rebuild_tables(Engine* E) {
     E->patch_off[l] = (int)E->h_patchtab.size();
     for (auto& b : E->lev[l].patches) {
       // tile .w = index of the patch in the all-level patch table
+      const size_t t0 = E->h_tiles.size();
       tiles_of_box(b, l, (int)E->h_patchtab.size(), E->h_tiles);
+      if (any_absorb(E)) {
+        const AbsorbTables T = absorb_tables_host(E);
+        for (size_t q = t0; q < E->h_tiles.size(); ++q) {
+          int4& td = E->h_tiles[q];
+          td.z |= absorb_tile_mask(T, l, td.x, td.y, (td.z >> 8) & 0xff, (td.z >> 16) & 0xff, b) << 24;
+        }
+      }
       E->h_patchtab.push_back(b);
     }
     level_neighbours(E->h_tiles, E->lev[l].patches, E->tile_off[l], (int)E->h_tiles.size(), E->h_nbr);
@@ -2785,9 +2811,6 @@ static int rebuild_tables(Engine* E) {
   E->tables_on_device = true;
   return check_launch("engine tables");
 }
-
-static bool any_absorb(const Engine* E);
-static AbsorbTables absorb_tables(const Engine* E);
 
 static EosConst32 eos_const32(const enl_engine_config& c) {
   EosConst32 e;
@@ -3040,6 +3063,18 @@ static AbsorbTables absorb_tables(const Engine* E) {
   return T;
 }
 
+// The host's copy: the continuation tests and the extents (absorb_tile_mask).
+static AbsorbTables absorb_tables_host(const Engine* E) {
+  AbsorbTables T = absorb_tables(E);
+  for (int l = 0; l < kL; ++l)
+    for (int d = 0; d < 4; ++d) {
+      T.env[l][d] = nullptr;
+      T.envf[l][d] = nullptr;
+      T.cont[l][d] = E->h_cont[l][d].empty() ? nullptr : E->h_cont[l][d].data();
+    }
+  return T;
+}
+
 // Envelope tables of every level, host-computed with the reference's formula
 // 1 - exp(-ln2 / w^2 * d^2) and the level's cell centres.
 static int build_absorb_tables(Engine* E) {
@@ -3079,6 +3114,7 @@ static int build_absorb_tables(Engine* E) {
       cudaMemcpy(E->d_env[l][d], h.data(), n[d] * sizeof(double), cudaMemcpyHostToDevice);
       cudaMemcpy(E->d_envf[l][d], hf.data(), n[d] * sizeof(float), cudaMemcpyHostToDevice);
       cudaMemcpy(E->d_cont[l][d], hc.data(), n[d], cudaMemcpyHostToDevice);
+      E->h_cont[l][d] = hc;
     }
   }
   return ENL_OK;
