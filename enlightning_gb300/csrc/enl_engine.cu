@@ -72,15 +72,6 @@ constexpr int kPlanesBytes = align128((kPlOffG + 5 * kPlaneG) * 4);   // 19840
 #define ENL_STAGE_UN_TMA 0
 #endif
 constexpr bool kUnTma = ENL_STAGE_UN_TMA != 0;
-// FP32 storage without staged u^n: prefetch (to L2) the u^n and H0 values of
-// each thread's cell when its tile starts.  Measured on the 3-level line
-// source: hybrid 0.342 ms per launch against 0.349 ms without.
-#ifndef ENL_PREFETCH_UN
-#define ENL_PREFETCH_UN 1
-#endif
-#ifndef ENL_PREFETCH_OP
-#define ENL_PREFETCH_OP "prefetch.global.L2"
-#endif
 constexpr int kUnBytes = 5 * kTH * kBW32 * 4;    // 6400
 constexpr int kH0Bytes = kTH * kBW32 * 4;        // 1280
 constexpr int kBufS = kTile32Bytes + (kUnTma ? kUnBytes + kH0Bytes : 0);  // per staging buffer
@@ -419,8 +410,7 @@ __device__ __forceinline__ bool uniform_maybe(const S* box) {
 // keeps its registers) around one block barrier in the kernel.  uniform_probe:
 // this thread's part: warp k < 7 holds field k of the box against its first
 // element, 16 bytes at a time, and every cell's u^n and H0 must equal those of
-// the tile's first cell (both loaded before the tile's wait; zero in stage 1
-// for u^n, which is the staged box).  uniform_hit, after the barrier's AND of
+// the tile's first cell (zero in stage 1 for u^n, which is the staged box).  uniform_hit, after the barrier's AND of
 // the probes: 1 when the level's cache entry holds the tile's inputs (the
 // cached outputs are stored into every cell of the tile and counted); 2 when
 // the tile must be computed (the caller's cell (0, 0) then fills the entry).
@@ -782,39 +772,20 @@ __global__ void __launch_bounds__(256, std::is_same<S, float>::value ? kStageBlo
     const int i0 = td.x, j0 = td.y;
     const int tx = lane, ty = warp;
     const bool valid = tx < w && ty < h;
-    // u^n and H0 of this thread's cell and of the tile's first cell, for the
-    // uniform-tile test: loaded before the wait, so that their latency
-    // overlaps it
-    S un_c[5] = {S(0), S(0), S(0), S(0), S(0)}, h0_c = S(0);
-    S un_f[5] = {S(0), S(0), S(0), S(0), S(0)}, h0_f = S(0);
-    if (A.uniform) {
-      const long g0 = (long)(j0 + 3) * A.pitch[lvl] + (i0 + 3);
-      const long g = valid ? g0 + (long)ty * A.pitch[lvl] + tx : g0;
-      h0_c = static_cast<const S*>(A.h0[lvl])[g];
-      h0_f = static_cast<const S*>(A.h0[lvl])[g0];
-      if (!A.un_is_in)
+    // u^n and H0 of this thread's cell are read in the epilogue, or by the
+    // uniform-tile test: start their way towards the SM now.  (Loading them
+    // here for the test cost more than it hid: with the registers this kernel
+    // has, the values went to the stack, and the block sat out their latency
+    // before the tile's own wait.)
+    if (valid && !kUnTma) {
+      const long g = (long)(j0 + ty + 3) * A.pitch[lvl] + (i0 + tx + 3);
+      asm volatile("prefetch.global.L2 [%0];" ::"l"(static_cast<const S*>(A.h0[lvl]) + g));
+      if (!A.un_is_in) {
+        const S* up = static_cast<const S*>(A.un[lvl]) + g;
 #pragma unroll
-        for (int k = 0; k < 5; ++k) {
-          un_c[k] = static_cast<const S*>(A.un[lvl])[k * A.fstride[lvl] + g];
-          un_f[k] = static_cast<const S*>(A.un[lvl])[k * A.fstride[lvl] + g0];
-        }
-    }
-#if ENL_PREFETCH_UN
-    if constexpr (kF32S && !kUnTma) {
-      // u^n and H0 of this thread's cell are read in the epilogue: start
-      // their way towards the SM now
-      if (!A.uniform && valid) {
-        const long g = (long)(j0 + ty + 3) * A.pitch[lvl] + (i0 + tx + 3);
-        const float* h0p = static_cast<const float*>(A.h0[lvl]) + g;
-        asm volatile(ENL_PREFETCH_OP " [%0];" ::"l"(h0p));
-        if (!A.un_is_in) {
-          const float* up = static_cast<const float*>(A.un[lvl]) + g;
-#pragma unroll
-          for (int k = 0; k < 5; ++k) asm volatile(ENL_PREFETCH_OP " [%0];" ::"l"(up + k * A.fstride[lvl]));
-        }
+        for (int k = 0; k < 5; ++k) asm volatile("prefetch.global.L2 [%0];" ::"l"(up + k * A.fstride[lvl]));
       }
     }
-#endif
     if (!mbar_wait_timed(&mbar[b], phase[b], kWaitNs)) {
       if (tid == 0) raise_health(A.health, ENL_ERR_TIMEOUT);
       // let copies in flight land (bounded) before the block leaves
@@ -832,6 +803,17 @@ __global__ void __launch_bounds__(256, std::is_same<S, float>::value ? kStageBlo
     if (A.uniform) {
       const S* box = reinterpret_cast<const S*>(dst[b]);
       if (uniform_maybe<S, kPl, kF32S ? kBW32 : kBW>(box)) {
+        // u^n and H0 of this thread's cell and of the tile's first cell
+        S un_c[5] = {S(0), S(0), S(0), S(0), S(0)}, un_f[5] = {S(0), S(0), S(0), S(0), S(0)};
+        const long g0 = (long)(j0 + 3) * A.pitch[lvl] + (i0 + 3);
+        const long g = valid ? g0 + (long)ty * A.pitch[lvl] + tx : g0;
+        const S h0_c = static_cast<const S*>(A.h0[lvl])[g], h0_f = static_cast<const S*>(A.h0[lvl])[g0];
+        if (!A.un_is_in)
+#pragma unroll
+          for (int k = 0; k < 5; ++k) {
+            un_c[k] = static_cast<const S*>(A.un[lvl])[k * A.fstride[lvl] + g];
+            un_f[k] = static_cast<const S*>(A.un[lvl])[k * A.fstride[lvl] + g0];
+          }
         const bool ok = uniform_probe<S, kPl, kF32S ? kBW32 : kBW>(box, s_first, w, h, un_c[0], un_c[1], un_c[2],
                                                                    un_c[3], un_c[4], h0_c, un_f[0], un_f[1], un_f[2],
                                                                    un_f[3], un_f[4], h0_f);
