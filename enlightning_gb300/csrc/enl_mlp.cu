@@ -6,6 +6,7 @@
 // below 0.9999.  The learned sensor predicts from 40 stencil features
 // (enl_mlp.cuh) whether WENO is needed, trained on the plain switch and on
 // the local difference between the DRP and WENO right-hand sides.
+#include <cstddef>
 #include <cstring>
 #include <cstdio>
 
@@ -16,107 +17,192 @@ namespace enl {
 
 // ---------------------------------------------------------------------------
 // Training: one block of 4 warps handles chunks of 64 samples (16 per warp).
+//
+// The six matrix products of a chunk are small (64 x 48 x 64 and 64 x 64 x 64),
+// so what bounds the kernel is everything around them: operand loads, the
+// activations and the reductions over samples.
+//   * Every fragment comes from shared memory by ldmatrix (four 8 x 8 tiles per
+//     instruction, transposed where the product runs over samples) from
+//     conflict-free padded rows; W2 is kept once, its transpose read from it.
+//   * GELU and its derivative are evaluated together, once per activation.
+//   * Bias gradients are a product with a row of ones on the tensor cores,
+//     done by the warp that has no rows of dW1, and dw3 is accumulated in
+//     registers; one warp summing 64 samples column by column kept the other
+//     three waiting.
+//   * As many blocks as fit (no second wave that stages the parameters again),
+//     features read 16 bytes at a time.
+// 65,536 samples: 84 -> 56 us a call (with its two clears).
 // ---------------------------------------------------------------------------
 constexpr int kChunk = 64;
 
-struct TrainSmem {
-  MlpSmem S;
-  __nv_bfloat16 w2[kHid][kHid];  // W2 [k][n] (B operand of dH1 = dZ2 W2^T)
-  __nv_bfloat16 xs[kChunk][kFeatPad];
-  __nv_bfloat16 h1[kChunk][kHid];
-  __nv_bfloat16 h2[kChunk][kHid];
-  __nv_bfloat16 dz1[kChunk][kHid];
-  __nv_bfloat16 dz2[kChunk][kHid];
-  float dl[kChunk];
+// (every matrix starts and every row lies on 16 bytes: ldmatrix and the wide
+// copies need it)
+struct alignas(16) TrainSmem {
+  alignas(16) MlpSmem S;
+  alignas(16) __nv_bfloat16 xs[kChunk][kLdF];
+  alignas(16) __nv_bfloat16 h1[kChunk][kLdH];
+  alignas(16) __nv_bfloat16 dz1[kChunk][kLdH];
+  alignas(16) __nv_bfloat16 dz2[kChunk][kLdH];
 };
+static_assert(offsetof(MlpSmem, w1t) % 16 == 0 && offsetof(MlpSmem, w2t) % 16 == 0 && offsetof(TrainSmem, xs) % 16 == 0 &&
+                  offsetof(TrainSmem, h1) % 16 == 0 && offsetof(TrainSmem, dz1) % 16 == 0 &&
+                  offsetof(TrainSmem, dz2) % 16 == 0 && kLdF * 2 % 16 == 0 && kLdH * 2 % 16 == 0,
+              "16-byte rows");
 
-__device__ __forceinline__ uint32_t pack_two(const __nv_bfloat16 lo, const __nv_bfloat16 hi) {
-  __nv_bfloat162 v;
-  v.x = lo;
-  v.y = hi;
-  return *reinterpret_cast<uint32_t*>(&v);
+// GELU and its derivative: Phi(x) by erf_as, whose exponential is the
+// density's, exp(-x^2 / 2).
+__device__ __forceinline__ void gelu_both(float x, float& g, float& d) {
+  g = gelu(x);
+  d = gelu_grad(x);
 }
 
-__global__ void __launch_bounds__(128) mlp_grad_kernel(const __nv_bfloat16* __restrict__ X,
-                                                       const float* __restrict__ y, const float* __restrict__ wgt,
-                                                       long N, const float* __restrict__ P, float* grad,
-                                                       double* loss_sum) {
+// C (16 x 64, n-tiles of 8) += A (16 x 16 fragment) B, B's 16 x 64 slice at p
+// stored [k][n] (rows of ld).
+__device__ __forceinline__ void mma_row64(float c[8][4], const uint32_t a[4], const __nv_bfloat16* p, int ld,
+                                          int lane) {
+  const __nv_bfloat16* q = p + (lane & 15) * ld + (lane >> 4) * 8;
+#pragma unroll
+  for (int n = 0; n < 8; n += 2) {
+    uint32_t b[4];
+    ldsm4t(b, q + n * 8);
+    mma_bf16(c[n], a[0], a[1], a[2], a[3], b[0], b[1]);
+    mma_bf16(c[n + 1], a[0], a[1], a[2], a[3], b[2], b[3]);
+  }
+}
+// The same with B stored [n][k].
+__device__ __forceinline__ void mma_col64(float c[8][4], const uint32_t a[4], const __nv_bfloat16* p, int ld,
+                                          int lane) {
+  const __nv_bfloat16* q = p + ((lane >> 4) * 8 + (lane & 7)) * ld + ((lane >> 3) & 1) * 8;
+#pragma unroll
+  for (int n = 0; n < 8; n += 2) {
+    uint32_t b[4];
+    ldsm4(b, q + n * 8 * ld);
+    mma_bf16(c[n], a[0], a[1], a[2], a[3], b[0], b[1]);
+    mma_bf16(c[n + 1], a[0], a[1], a[2], a[3], b[2], b[3]);
+  }
+}
+
+__device__ __forceinline__ float2 bf16_pair(uint32_t v) {
+  return __bfloat1622float2(*reinterpret_cast<const __nv_bfloat162*>(&v));
+}
+
+__global__ void __launch_bounds__(128, 3) mlp_grad_kernel(const __nv_bfloat16* __restrict__ X,
+                                                          const float* __restrict__ y, const float* __restrict__ wgt,
+                                                          long N, const float* __restrict__ P, float* grad,
+                                                          double* loss_sum) {
   extern __shared__ __align__(16) unsigned char sm_raw[];
   TrainSmem& T = *reinterpret_cast<TrainSmem*>(sm_raw);
   const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
   const int g = lane >> 2, t = lane & 3;
   mlp_stage_params(T.S, P, tid, 128);
-  for (int e = tid; e < kHid * kHid; e += 128) {
-    int k = e / kHid, n = e % kHid;
-    T.w2[k][n] = __float2bfloat16_rn(P[kOffW2 + k * kHid + n]);
-  }
-  // per-thread accumulators of the block's weight gradients
+  for (int e = tid; e < kChunk * (kFeatPad - kFeat); e += 128)
+    T.xs[e / (kFeatPad - kFeat)][kFeat + e % (kFeatPad - kFeat)] = __float2bfloat16_rn(0.0f);
+  const bool wide = (reinterpret_cast<uintptr_t>(X) & 15) == 0;
+  // the block's weight gradients: rows 16 warp .. of dW2; of dW1 (warps 0-2)
+  // or, warp 3, db1 in row 0 and db2 in row 8 of products with ones
   float aw2[8][4], aw1[8][4];
+  float aw3[8][2], ab3 = 0.f;
 #pragma unroll
-  for (int n = 0; n < 8; ++n)
+  for (int n = 0; n < 8; ++n) {
 #pragma unroll
     for (int q = 0; q < 4; ++q) aw2[n][q] = aw1[n][q] = 0.f;
-  float ab1[2] = {0.f, 0.f}, ab2[2] = {0.f, 0.f}, aw3[2] = {0.f, 0.f}, ab3 = 0.f;
+    aw3[n][0] = aw3[n][1] = 0.f;
+  }
+  // A fragments with ones in row 0 and in row 8
+  const uint32_t one = g == 0 ? 0x3f803f80u : 0u;
+  const uint32_t ones0[4] = {one, 0u, one, 0u}, ones8[4] = {0u, one, 0u, one};
   double lsum = 0.0;
-  __syncthreads();
   for (long c0 = (long)blockIdx.x * kChunk; c0 < N; c0 += (long)gridDim.x * kChunk) {
-    for (int e = tid; e < kChunk * kFeatPad; e += 128) {
-      int r = e / kFeatPad, k = e % kFeatPad;
-      long s = c0 + r;
-      T.xs[r][k] = (s < N && k < kFeat) ? X[s * kFeat + k] : __float2bfloat16_rn(0.0f);
+    if (wide && c0 + kChunk <= N) {
+      const uint4* src = reinterpret_cast<const uint4*>(X + c0 * kFeat);
+      for (int e = tid; e < kChunk * kFeat / 8; e += 128) {
+        const int r = e / (kFeat / 8), q = e % (kFeat / 8);
+        *reinterpret_cast<uint4*>(&T.xs[r][8 * q]) = src[e];
+      }
+    } else {
+      for (int e = tid; e < kChunk * kFeat; e += 128) {
+        const int r = e / kFeat, k = e % kFeat;
+        T.xs[r][k] = c0 + r < N ? X[(c0 + r) * kFeat + k] : __float2bfloat16_rn(0.0f);
+      }
     }
     __syncthreads();
     // forward, 16 rows per warp
-    MlpFwd16 F;
-    mlp_forward16(T.S, &T.xs[warp * 16][0], kFeatPad, lane, F);
-    const int r0 = warp * 16 + g, r1 = r0 + 8;
+    const int r0 = warp * 16 + g, r1 = r0 + 8, arow = warp * 16 + (lane & 15), acol = (lane >> 4) * 8;
+    float z1[8][4];
+#pragma unroll
+    for (int n = 0; n < 8; ++n)
+#pragma unroll
+      for (int q = 0; q < 4; ++q) z1[n][q] = T.S.b1[n * 8 + 2 * t + (q & 1)];
+#pragma unroll
+    for (int kc = 0; kc < 3; ++kc) {
+      uint32_t a[4];
+      ldsm4(a, &T.xs[arow][kc * 16 + acol]);
+      mma_col64(z1, a, &T.S.w1t[0][kc * 16], kLdF, lane);
+    }
+    // hidden layer 1: BF16 A fragments of layer 2, kept for dW2; z1 becomes
+    // the derivative of the activation
+    float z2[8][4];
+#pragma unroll
+    for (int n = 0; n < 8; ++n)
+#pragma unroll
+      for (int q = 0; q < 4; ++q) z2[n][q] = T.S.b2[n * 8 + 2 * t + (q & 1)];
+#pragma unroll
+    for (int kc = 0; kc < 4; ++kc) {
+      uint32_t a[4];
+#pragma unroll
+      for (int half = 0; half < 2; ++half) {
+        const int n = 2 * kc + half, col = n * 8 + 2 * t;
+        float h[4];
+#pragma unroll
+        for (int q = 0; q < 4; ++q) gelu_both(z1[n][q], h[q], z1[n][q]);
+        a[2 * half] = pack_bf16(h[0], h[1]);
+        a[2 * half + 1] = pack_bf16(h[2], h[3]);
+        *reinterpret_cast<uint32_t*>(&T.h1[r0][col]) = a[2 * half];
+        *reinterpret_cast<uint32_t*>(&T.h1[r1][col]) = a[2 * half + 1];
+      }
+      mma_col64(z2, a, &T.S.w2t[0][kc * 16], kLdH, lane);
+    }
+    // last layer: hidden activations rounded to BF16 like the tensor-core
+    // layers' inputs; z2 becomes the derivative
+    float s0 = 0.f, s1 = 0.f;
+    uint32_t h2[8][2];
 #pragma unroll
     for (int n = 0; n < 8; ++n) {
-      int col = n * 8 + 2 * t;
-      T.h1[r0][col] = __float2bfloat16_rn(gelu(F.z1[n][0]));
-      T.h1[r0][col + 1] = __float2bfloat16_rn(gelu(F.z1[n][1]));
-      T.h1[r1][col] = __float2bfloat16_rn(gelu(F.z1[n][2]));
-      T.h1[r1][col + 1] = __float2bfloat16_rn(gelu(F.z1[n][3]));
-      T.h2[r0][col] = __float2bfloat16_rn(gelu(F.z2[n][0]));
-      T.h2[r0][col + 1] = __float2bfloat16_rn(gelu(F.z2[n][1]));
-      T.h2[r1][col] = __float2bfloat16_rn(gelu(F.z2[n][2]));
-      T.h2[r1][col + 1] = __float2bfloat16_rn(gelu(F.z2[n][3]));
+      const int col = n * 8 + 2 * t;
+      float h[4];
+#pragma unroll
+      for (int q = 0; q < 4; ++q) gelu_both(z2[n][q], h[q], z2[n][q]);
+      h2[n][0] = pack_bf16(h[0], h[1]);
+      h2[n][1] = pack_bf16(h[2], h[3]);
+      const float2 u = bf16_pair(h2[n][0]), v = bf16_pair(h2[n][1]);
+      s0 += u.x * T.S.w3[col] + u.y * T.S.w3[col + 1];
+      s1 += v.x * T.S.w3[col] + v.y * T.S.w3[col + 1];
     }
-    // BCE-with-logits gradient of rows r0, r1 (lanes t == 0 hold the logits)
+    s0 += __shfl_xor_sync(0xffffffffu, s0, 1);
+    s0 += __shfl_xor_sync(0xffffffffu, s0, 2);
+    s1 += __shfl_xor_sync(0xffffffffu, s1, 1);
+    s1 += __shfl_xor_sync(0xffffffffu, s1, 2);
+    // BCE-with-logits gradient of rows r0, r1 (lanes t == 0)
     float dl0 = 0.f, dl1 = 0.f;
     if (t == 0) {
-      long s0 = c0 + r0, s1 = c0 + r1;
-      float z0 = F.logit[0], z1 = F.logit[1];
-      if (s0 < N) {
-        float w = wgt[s0], yy = y[s0];
-        dl0 = w * (1.0f / (1.0f + __expf(-z0)) - yy);
-        lsum += (double)(w * (fmaxf(z0, 0.f) - yy * z0 + log1pf(__expf(-fabsf(z0)))));
+      const long i0 = c0 + r0, i1 = c0 + r1;
+      const float l0 = s0 + T.S.b3, l1 = s1 + T.S.b3;
+      if (i0 < N) {
+        const float w = wgt[i0], yy = y[i0];
+        dl0 = w * (1.0f / (1.0f + __expf(-l0)) - yy);
+        lsum += (double)(w * (fmaxf(l0, 0.f) - yy * l0 + log1pf(__expf(-fabsf(l0)))));
       }
-      if (s1 < N) {
-        float w = wgt[s1], yy = y[s1];
-        dl1 = w * (1.0f / (1.0f + __expf(-z1)) - yy);
-        lsum += (double)(w * (fmaxf(z1, 0.f) - yy * z1 + log1pf(__expf(-fabsf(z1)))));
+      if (i1 < N) {
+        const float w = wgt[i1], yy = y[i1];
+        dl1 = w * (1.0f / (1.0f + __expf(-l1)) - yy);
+        lsum += (double)(w * (fmaxf(l1, 0.f) - yy * l1 + log1pf(__expf(-fabsf(l1)))));
       }
-      T.dl[r0] = dl0;
-      T.dl[r1] = dl1;
+      ab3 += dl0 + dl1;
     }
     dl0 = __shfl_sync(0xffffffffu, dl0, lane & ~3);
     dl1 = __shfl_sync(0xffffffffu, dl1, lane & ~3);
-    // dZ2 = (dl w3) * gelu'(z2), C-fragment layout
-    float dz2[8][4];
-#pragma unroll
-    for (int n = 0; n < 8; ++n) {
-      int col = n * 8 + 2 * t;
-      dz2[n][0] = dl0 * T.S.w3[col] * gelu_grad(F.z2[n][0]);
-      dz2[n][1] = dl0 * T.S.w3[col + 1] * gelu_grad(F.z2[n][1]);
-      dz2[n][2] = dl1 * T.S.w3[col] * gelu_grad(F.z2[n][2]);
-      dz2[n][3] = dl1 * T.S.w3[col + 1] * gelu_grad(F.z2[n][3]);
-      T.dz2[r0][col] = __float2bfloat16_rn(dz2[n][0]);
-      T.dz2[r0][col + 1] = __float2bfloat16_rn(dz2[n][1]);
-      T.dz2[r1][col] = __float2bfloat16_rn(dz2[n][2]);
-      T.dz2[r1][col + 1] = __float2bfloat16_rn(dz2[n][3]);
-    }
-    // dH1 = dZ2 W2^T on the tensor cores (A = dZ2 from registers)
+    // dw3, and dZ2 = (dl w3) gelu'(z2) as A fragments and in shared memory;
+    // dH1 = dZ2 W2^T on the tensor cores
     float dh1[8][4];
 #pragma unroll
     for (int n = 0; n < 8; ++n)
@@ -124,76 +210,46 @@ __global__ void __launch_bounds__(128) mlp_grad_kernel(const __nv_bfloat16* __re
       for (int q = 0; q < 4; ++q) dh1[n][q] = 0.f;
 #pragma unroll
     for (int kc = 0; kc < 4; ++kc) {
-      uint32_t a0 = pack_bf16(dz2[2 * kc][0], dz2[2 * kc][1]);
-      uint32_t a1 = pack_bf16(dz2[2 * kc][2], dz2[2 * kc][3]);
-      uint32_t a2 = pack_bf16(dz2[2 * kc + 1][0], dz2[2 * kc + 1][1]);
-      uint32_t a3 = pack_bf16(dz2[2 * kc + 1][2], dz2[2 * kc + 1][3]);
+      uint32_t a[4];
 #pragma unroll
-      for (int n = 0; n < 8; ++n) {
-        // B(kk = hidden-2 index, col = hidden-1 index) = W2[col][kk]
-        uint32_t b0 = ld_pair(&T.w2[n * 8 + g][kc * 16 + 2 * t]);
-        uint32_t b1 = ld_pair(&T.w2[n * 8 + g][kc * 16 + 2 * t + 8]);
-        mma_bf16(dh1[n], a0, a1, a2, a3, b0, b1);
+      for (int half = 0; half < 2; ++half) {
+        const int n = 2 * kc + half, col = n * 8 + 2 * t;
+        const float2 u = bf16_pair(h2[n][0]), v = bf16_pair(h2[n][1]);
+        aw3[n][0] += dl0 * u.x + dl1 * v.x;
+        aw3[n][1] += dl0 * u.y + dl1 * v.y;
+        const float w0 = T.S.w3[col], w1 = T.S.w3[col + 1];
+        a[2 * half] = pack_bf16(dl0 * w0 * z2[n][0], dl0 * w1 * z2[n][1]);
+        a[2 * half + 1] = pack_bf16(dl1 * w0 * z2[n][2], dl1 * w1 * z2[n][3]);
+        *reinterpret_cast<uint32_t*>(&T.dz2[r0][col]) = a[2 * half];
+        *reinterpret_cast<uint32_t*>(&T.dz2[r1][col]) = a[2 * half + 1];
       }
+      // B(kk = hidden-2 index, col = hidden-1 index) = W2[col][kk] = w2t[kk][col]
+      mma_row64(dh1, a, &T.S.w2t[kc * 16][0], kLdH, lane);
     }
 #pragma unroll
     for (int n = 0; n < 8; ++n) {
-      int col = n * 8 + 2 * t;
-      T.dz1[r0][col] = __float2bfloat16_rn(dh1[n][0] * gelu_grad(F.z1[n][0]));
-      T.dz1[r0][col + 1] = __float2bfloat16_rn(dh1[n][1] * gelu_grad(F.z1[n][1]));
-      T.dz1[r1][col] = __float2bfloat16_rn(dh1[n][2] * gelu_grad(F.z1[n][2]));
-      T.dz1[r1][col + 1] = __float2bfloat16_rn(dh1[n][3] * gelu_grad(F.z1[n][3]));
+      const int col = n * 8 + 2 * t;
+      *reinterpret_cast<uint32_t*>(&T.dz1[r0][col]) = pack_bf16(dh1[n][0] * z1[n][0], dh1[n][1] * z1[n][1]);
+      *reinterpret_cast<uint32_t*>(&T.dz1[r1][col]) = pack_bf16(dh1[n][2] * z1[n][2], dh1[n][3] * z1[n][3]);
     }
     __syncthreads();
-    // weight gradients, reduction over the 64 samples on the tensor cores:
+    // weight gradients, sums over the 64 samples on the tensor cores:
     // dW2[k][n] = sum_s H1[s][k] dZ2[s][n] (warp w: rows k of m-tile w)
     // dW1[k][n] = sum_s X[s][k] dZ1[s][n]  (warps 0-2: m-tiles of k < 48)
+    // db2[n], db1[n] = sum_s dZ2[s][n], dZ1[s][n] (warp 3: ones in place of A)
+    const int trow = ((lane >> 4) & 1) * 8 + (lane & 7), tcol = warp * 16 + ((lane >> 3) & 1) * 8;
 #pragma unroll
     for (int ks = 0; ks < 4; ++ks) {
-      const int s0 = ks * 16 + 2 * t;
-      const int m0 = warp * 16 + g;
-      uint32_t a0 = pack_two(T.h1[s0][m0], T.h1[s0 + 1][m0]);
-      uint32_t a1 = pack_two(T.h1[s0][m0 + 8], T.h1[s0 + 1][m0 + 8]);
-      uint32_t a2 = pack_two(T.h1[s0 + 8][m0], T.h1[s0 + 9][m0]);
-      uint32_t a3 = pack_two(T.h1[s0 + 8][m0 + 8], T.h1[s0 + 9][m0 + 8]);
-#pragma unroll
-      for (int n = 0; n < 8; ++n) {
-        const int nn = n * 8 + g;
-        uint32_t b0 = pack_two(T.dz2[s0][nn], T.dz2[s0 + 1][nn]);
-        uint32_t b1 = pack_two(T.dz2[s0 + 8][nn], T.dz2[s0 + 9][nn]);
-        mma_bf16(aw2[n], a0, a1, a2, a3, b0, b1);
-      }
+      uint32_t a[4];
+      ldsm4t(a, &T.h1[ks * 16 + trow][tcol]);
+      mma_row64(aw2, a, &T.dz2[ks * 16][0], kLdH, lane);
       if (warp < 3) {
-        uint32_t c0_ = pack_two(T.xs[s0][m0], T.xs[s0 + 1][m0]);
-        uint32_t c1_ = pack_two(T.xs[s0][m0 + 8], T.xs[s0 + 1][m0 + 8]);
-        uint32_t c2_ = pack_two(T.xs[s0 + 8][m0], T.xs[s0 + 9][m0]);
-        uint32_t c3_ = pack_two(T.xs[s0 + 8][m0 + 8], T.xs[s0 + 9][m0 + 8]);
-#pragma unroll
-        for (int n = 0; n < 8; ++n) {
-          const int nn = n * 8 + g;
-          uint32_t b0 = pack_two(T.dz1[s0][nn], T.dz1[s0 + 1][nn]);
-          uint32_t b1 = pack_two(T.dz1[s0 + 8][nn], T.dz1[s0 + 9][nn]);
-          mma_bf16(aw1[n], c0_, c1_, c2_, c3_, b0, b1);
-        }
+        ldsm4t(a, &T.xs[ks * 16 + trow][tcol]);
+        mma_row64(aw1, a, &T.dz1[ks * 16][0], kLdH, lane);
+      } else {
+        mma_row64(aw1, ones0, &T.dz1[ks * 16][0], kLdH, lane);
+        mma_row64(aw1, ones8, &T.dz2[ks * 16][0], kLdH, lane);
       }
-    }
-    // bias and last-layer gradients on the CUDA cores (2 columns per lane)
-    if (warp == 3) {
-#pragma unroll
-      for (int h = 0; h < 2; ++h) {
-        int col = lane * 2 + h;
-        float sb1 = 0.f, sb2 = 0.f, sw3 = 0.f;
-        for (int s = 0; s < kChunk; ++s) {
-          sb1 += __bfloat162float(T.dz1[s][col]);
-          sb2 += __bfloat162float(T.dz2[s][col]);
-          sw3 += T.dl[s] * __bfloat162float(T.h2[s][col]);
-        }
-        ab1[h] += sb1;
-        ab2[h] += sb2;
-        aw3[h] += sw3;
-      }
-      if (lane == 0)
-        for (int s = 0; s < kChunk; ++s) ab3 += T.dl[s];
     }
     __syncthreads();
   }
@@ -215,17 +271,23 @@ __global__ void __launch_bounds__(128) mlp_grad_kernel(const __nv_bfloat16* __re
         atomicAdd(&grad[kOffW1 + k1 * kHid + col], aw1[n][2]);
         atomicAdd(&grad[kOffW1 + k1 * kHid + col + 1], aw1[n][3]);
       }
+    } else if (g == 0) {  // rows 0 and 8
+      atomicAdd(&grad[kOffB1 + col], aw1[n][0]);
+      atomicAdd(&grad[kOffB1 + col + 1], aw1[n][1]);
+      atomicAdd(&grad[kOffB2 + col], aw1[n][2]);
+      atomicAdd(&grad[kOffB2 + col + 1], aw1[n][3]);
     }
-  }
-  if (warp == 3) {
 #pragma unroll
-    for (int h = 0; h < 2; ++h) {
-      atomicAdd(&grad[kOffB1 + lane * 2 + h], ab1[h]);
-      atomicAdd(&grad[kOffB2 + lane * 2 + h], ab2[h]);
-      atomicAdd(&grad[kOffW3 + lane * 2 + h], aw3[h]);
+    for (int q = 0; q < 2; ++q) {
+      float v = aw3[n][q];
+#pragma unroll
+      for (int o = 4; o < 32; o <<= 1) v += __shfl_xor_sync(0xffffffffu, v, o);
+      if (g == 0) atomicAdd(&grad[kOffW3 + col + q], v);
     }
-    if (lane == 0) atomicAdd(&grad[kOffB3], ab3);
   }
+#pragma unroll
+  for (int o = 4; o < 32; o <<= 1) ab3 += __shfl_xor_sync(0xffffffffu, ab3, o);
+  if (lane == 0) atomicAdd(&grad[kOffB3], ab3);
   if (loss_sum) {
     for (int o = 16; o > 0; o >>= 1) lsum += __shfl_xor_sync(0xffffffffu, lsum, o);
     if (lane == 0) atomicAdd(loss_sum, lsum);
@@ -236,7 +298,7 @@ __global__ void __launch_bounds__(128) mlp_grad_kernel(const __nv_bfloat16* __re
 __global__ void __launch_bounds__(128) mlp_forward_kernel(const __nv_bfloat16* __restrict__ X, long N,
                                                           const float* __restrict__ P, float* __restrict__ logit) {
   __shared__ MlpSmem S;
-  __shared__ __align__(16) __nv_bfloat16 xs[kChunk][kFeatPad];
+  __shared__ __align__(16) __nv_bfloat16 xs[kChunk][kLdF];
   const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
   mlp_stage_params(S, P, tid, 128);
   __syncthreads();
@@ -248,7 +310,7 @@ __global__ void __launch_bounds__(128) mlp_forward_kernel(const __nv_bfloat16* _
     }
     __syncthreads();
     MlpFwd16 F;
-    mlp_forward16(S, &xs[warp * 16][0], kFeatPad, lane, F);
+    mlp_forward16(S, &xs[warp * 16][0], kLdF, lane, F);
     if ((lane & 3) == 0) {
       long s0 = c0 + warp * 16 + (lane >> 2);
       if (s0 < N) logit[s0] = F.logit[0];
@@ -326,7 +388,7 @@ int enl_mlp_grad(const void* X, const float* y, const float* wgt, long n, const 
   int nsm = 148;
   cudaDeviceGetAttribute(&nsm, cudaDevAttrMultiProcessorCount, 0);
   long chunks = (n + kChunk - 1) / kChunk;
-  int blocks = (int)std::min<long>(chunks, (long)nsm * 4);
+  int blocks = (int)std::min<long>(chunks, (long)nsm * 3);  // resident at once
   mlp_grad_kernel<<<blocks, 128, sizeof(TrainSmem), stream()>>>((const __nv_bfloat16*)X, y, wgt, n, params, grad,
                                                                loss_sum);
   return check_launch("mlp_grad");

@@ -25,10 +25,14 @@ constexpr int kOffW3 = kOffB2 + kHid;           // w3[k]
 constexpr int kOffB3 = kOffW3 + kHid;
 constexpr int kNParams = kOffB3 + 1;            // 6849
 
+// Rows of the BF16 matrices, padded by 16 bytes: the eight rows that a
+// fragment load touches at once then lie in different shared-memory banks
+// (rows of 128 bytes put them all in the same four).
+constexpr int kLdF = kFeatPad + 8, kLdH = kHid + 8;
 // Shared-memory image of the network (BF16 transposed matrices + FP32 vectors).
 struct MlpSmem {
-  __nv_bfloat16 w1t[kHid][kFeatPad];  // [n][k], k >= 40 zero
-  __nv_bfloat16 w2t[kHid][kHid];      // [n][k]
+  __nv_bfloat16 w1t[kHid][kLdF];  // [n][k], k >= 40 zero
+  __nv_bfloat16 w2t[kHid][kLdH];  // [n][k]
   float b1[kHid], b2[kHid], w3[kHid];
   float b3;
 };
@@ -50,14 +54,12 @@ inline void mlp_build_image(const float* P, MlpSmem& S) {
 }
 
 __device__ __forceinline__ void mlp_stage_params(MlpSmem& S, const float* __restrict__ P, int tid, int nthr) {
+  // (neighbouring threads read neighbouring parameters)
   for (int e = tid; e < kHid * kFeatPad; e += nthr) {
-    int n = e / kFeatPad, k = e % kFeatPad;
-    S.w1t[n][k] = __float2bfloat16_rn(k < kFeat ? P[kOffW1 + k * kHid + n] : 0.0f);
+    const int k = e / kHid, n = e % kHid;
+    S.w1t[n][k] = __float2bfloat16_rn(k < kFeat ? P[kOffW1 + e] : 0.0f);
   }
-  for (int e = tid; e < kHid * kHid; e += nthr) {
-    int n = e / kHid, k = e % kHid;
-    S.w2t[n][k] = __float2bfloat16_rn(P[kOffW2 + k * kHid + n]);
-  }
+  for (int e = tid; e < kHid * kHid; e += nthr) S.w2t[e % kHid][e / kHid] = __float2bfloat16_rn(P[kOffW2 + e]);
   for (int e = tid; e < kHid; e += nthr) {
     S.b1[e] = P[kOffB1 + e];
     S.b2[e] = P[kOffB2 + e];
@@ -97,6 +99,21 @@ __device__ __forceinline__ float erf_as(float x) {
       t * fmaf(t, fmaf(t, fmaf(t, fmaf(t, 1.061405429f, -1.453152027f), 1.421413741f), -0.284496736f), 0.254829592f);
   return copysignf(fmaf(-poly, __expf(-ax * ax), 1.0f), x);
 }
+// Fragments of four 8 x 8 BF16 tiles, one row address per lane (lanes 8 q ..
+// 8 q + 7: the rows of tile q); T transposed.
+__device__ __forceinline__ void ldsm4(uint32_t r[4], const __nv_bfloat16* p) {
+  const uint32_t a = (uint32_t)__cvta_generic_to_shared(p);
+  asm volatile("ldmatrix.sync.aligned.m8n8.x4.shared.b16 {%0,%1,%2,%3}, [%4];"
+               : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3])
+               : "r"(a));
+}
+__device__ __forceinline__ void ldsm4t(uint32_t r[4], const __nv_bfloat16* p) {
+  const uint32_t a = (uint32_t)__cvta_generic_to_shared(p);
+  asm volatile("ldmatrix.sync.aligned.m8n8.x4.trans.shared.b16 {%0,%1,%2,%3}, [%4];"
+               : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3])
+               : "r"(a));
+}
+
 __device__ __forceinline__ float gelu(float x) { return 0.5f * x * (1.0f + erf_as(x * 0.70710678118654752f)); }
 __device__ __forceinline__ float gelu_grad(float x) {
   // d/dx [x Phi(x)] = Phi(x) + x phi(x)
