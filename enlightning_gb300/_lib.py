@@ -34,8 +34,19 @@ SIGNATURES = {
     "enl_rhs": (i32, [i32] + [i32] * 6 + [dp, dp, vp, i64, i64, vp, vp, i64, i64, vp, vp]
                 + [f64] * 7 + [dp, i32, f64, f64, vp]),
     "enl_phys_bc": (i32, [i32] * 6 + [ip, ip, i32, i32, vp, vp, vp, vp]),
+    "enl_patch_stage": (i32, [vp, f64, f64, f64, f64, i32]),
     "enl_absorb": (i32, [i32] * 6 + [dp, dp, dp, dp, ip, f64, f64, f64, f64, vp, vp, vp]),
 }
+
+
+class PatchArgs(C.Structure):
+    """enl_patch: one patch and its parameters, for enl_patch_stage."""
+    _fields_ = ([("box", C.c_int * 4), ("gcw", C.c_int * 2), ("fill", C.c_int * 2), ("touches", C.c_int * 4),
+                 ("bc", C.c_int * 4), ("level", C.c_int), ("xlo", C.c_double * 2), ("dx", C.c_double * 2),
+                 ("grid_xlo", C.c_double * 2), ("grid_xhi", C.c_double * 2), ("tol", C.c_double * 3)]
+                + [(k, C.c_double) for k in ("weno_alpha", "kappa", "mu", "muB", "R", "T_star_n", "tau_n", "c", "c_lr",
+                                             "rho0", "gamma1", "c_p", "p0", "T0", "c_v", "absorb_width")]
+                + [(k, C.c_void_p) for k in ("w_n", "pressure", "temperature", "source_g", "w", "source", "rhs")])
 
 
 class EngineConfig(C.Structure):

@@ -131,23 +131,38 @@ class Enlightning:
                                      _lib.iarr(self.bc), p["bc_absorb_width"], p["p0"], p["T0"], p["rho0"],
                                      _ptr(P.w_scr), _ptr(P.pres), _ptr(P.temp)), "enl_absorb")
 
+    def _patch_args(self, P: Patch, absorb, ghosts):
+        """The patch and the strategy's parameters as enl_patch_stage takes
+        them; filled anew by every call, so changes of either are seen."""
+        p, g = self.p, P.g
+        a = _lib.PatchArgs()
+        a.box[:], a.gcw[:], a.fill[:] = P.box, (g, g), (g, g)
+        a.touches[:] = [int(t) for t in P.touches]
+        a.bc[:] = self.bc if absorb else [b if b != ABSORB else 0 for b in self.bc]
+        a.level = int(P.level)
+        a.xlo[:], a.dx[:], a.grid_xlo[:], a.grid_xhi[:] = P.xlo, P.dx, self.domain_xlo, self.domain_xhi
+        a.tol[:] = p["tol"]
+        a.weno_alpha, a.kappa, a.mu, a.muB, a.R = p["weno_alpha"], p["kappa"], p["mu"], p["muB"], p["R"]
+        a.T_star_n, a.tau_n, a.c, a.c_lr, a.rho0 = p["T_star_n"], p["tau_n"], p["c"], p["c_lr"], p["rho0"]
+        a.gamma1, a.c_p, a.p0, a.T0, a.c_v = p["gamma1"], p["c_p"], p["p0"], p["T0"], p["c_v"]
+        a.absorb_width = p["bc_absorb_width"]
+        a.w_n, a.pressure, a.temperature = _ptr(P.w_scr), _ptr(P.pres), _ptr(P.temp)
+        a.w, a.source, a.rhs = _ptr(P.w_cur), _ptr(P.src), _ptr(P.K)
+        if ghosts:
+            a.source_g = _ptr(P.src_g)
+        return a
+
+    def _stock(self, *names):
+        """True while the named methods are this class's own."""
+        return all(getattr(type(self), n) is _OWN[n] and n not in self.__dict__ for n in names)
+
     # -- enlightning::singleStep (enlightning.C:459-583) --------------------
     def single_step(self, P: Patch, dt: float, a1: float, a2: float, beta: float):
-        L, p, b, g = self.L, self.p, P.box, P.g
-        I = _lib.iref
-        D = _lib.dref
-        L.rhs_(I(b[0]), I(b[1]), I(b[2]), I(b[3]), I(g), I(g), _lib.darr(P.xlo), _lib.darr(P.dx),
-               _ptr(P.w_scr), _ptr(P.src), _ptr(P.K), _ptr(P.pres), _ptr(P.temp), D(p["weno_alpha"]),
-               D(p["kappa"]), D(p["mu"]), D(p["muB"]), D(p["R"]), D(p["T_star_n"]), D(p["T_star_o"]),
-               D(p["tau_n"]), D(p["tau_o"]), _lib.darr(p["tol"]), I(P.level), D(p["c"]), D(p["c_lr"]),
-               I(NEQU))
-        L.runge_kutta_(I(b[0]), I(b[1]), I(b[2]), I(b[3]), I(g), I(g), D(dt), D(a1), D(a2), D(beta),
-                       _ptr(P.w_scr), _ptr(P.w_cur), _ptr(P.K), I(NEQU))
-        L.update_state_(_lib.darr(P.dx), _lib.darr(P.xlo), I(b[0]), I(b[1]), I(b[2]), I(b[3]), I(g), I(g),
-                        _ptr(P.w_scr), _ptr(P.pres), _ptr(P.temp), D(p["rho0"]), D(p["c"]), D(p["gamma1"]),
-                        D(p["c_p"]), D(p["p0"]), D(p["T0"]), D(p["c_lr"]), D(p["c_v"]), D(p["R_tilde"]),
-                        D(p["M"]), D(p["R"]), I(NEQU))
-        self.set_absorbing_boundary_conditions(P)
+        stock = self._stock("set_absorbing_boundary_conditions")
+        a = self._patch_args(P, absorb=stock, ghosts=False)
+        self.L.enl_patch_stage(C.byref(a), dt, a1, a2, beta, 0)
+        if not stock:
+            self.set_absorbing_boundary_conditions(P)
         _lib.check_sticky("single_step")
 
     # -- enlightning::tagGradientDetectorCells (enlightning.C:586-628) ------
@@ -160,9 +175,22 @@ class Enlightning:
     # -- one MOL step of a single-patch hierarchy ---------------------------
     def advance(self, P: Patch, dt: float, nsteps: int = 1):
         a1s, a2s, bs = self.rk
+        # with this class's own ghost fill and stage, one library call per
+        # stage (a patch's arguments through ctypes took longer than a small
+        # patch's kernels); an override of either is called as before
+        stock = self._stock("set_physical_boundary_conditions", "set_absorbing_boundary_conditions", "single_step")
+        a = self._patch_args(P, absorb=True, ghosts=True) if stock else None
         for _ in range(nsteps):
             P.interior(P.w_scr).copy_(P.w_cur)          # copy current -> scratch
             for s in range(len(a1s)):
-                self.set_physical_boundary_conditions(P)
-                self.single_step(P, dt, a1s[s], a2s[s], bs[s])
+                if stock:
+                    self.L.enl_patch_stage(C.byref(a), dt, a1s[s], a2s[s], bs[s], 1)
+                    _lib.check_sticky("advance")
+                else:
+                    self.set_physical_boundary_conditions(P)
+                    self.single_step(P, dt, a1s[s], a2s[s], bs[s])
             P.w_cur.copy_(P.interior(P.w_scr))          # copy scratch -> current
+
+
+_OWN = {n: getattr(Enlightning, n)
+        for n in ("set_physical_boundary_conditions", "set_absorbing_boundary_conditions", "single_step")}

@@ -153,6 +153,27 @@ int enl_absorb(int ifirst0, int ilast0, int ifirst1, int ilast1, int gcw0,
                double absorb_width, double p0, double T0, double rho0,
                double* w_n, double* pressure, double* temperature);
 
+/* One RK stage of one patch, enlightning::singleStep (enlightning.C:459-583)
+ * and, with fill_ghosts, the ghost fill before it: enl_phys_bc, rhs_ with the
+ * scheme of enl_set_rhs_variant, then runge_kutta_, update_state_ and
+ * enl_absorb in one pass.  The same results as those calls one after another.
+ * Arrays as there (SAMRAI layout, device memory): w_n, pressure, temperature,
+ * source_g ghosted; w, source, rhs interior; source_g is read only with
+ * fill_ghosts. */
+typedef struct {
+  int box[4];             /* ifirst0, ilast0, ifirst1, ilast1                */
+  int gcw[2], fill[2];    /* ghost width; ghost width to fill                */
+  int touches[4], bc[4];  /* as enl_phys_bc, enl_absorb                      */
+  int level;
+  double xlo[2], dx[2], grid_xlo[2], grid_xhi[2], tol[3];
+  double weno_alpha, kappa, mu, muB, R, T_star_n, tau_n, c, c_lr;
+  double rho0, gamma1, c_p, p0, T0, c_v, absorb_width;
+  double *w_n, *pressure, *temperature, *source_g;
+  double *w, *source, *rhs;
+} enl_patch;
+int enl_patch_stage(const enl_patch* patch, double dt, double alpha_1,
+                    double alpha_2, double beta, int fill_ghosts);
+
 /* ====================================================================== */
 /* Part 3: batched multi-level engine                                      */
 /* ====================================================================== */
