@@ -797,7 +797,7 @@ KERNEL_NOTES = {
               "cells under their 2x2 stencils read",
     "physbc": "physical ghost band fill (sides a stencil reads): one read and one write per band cell",
     "coarsen": "fine-to-coarse averaging: ratio^2 fine reads + one coarse write per covered coarse cell",
-    "cfl": "CFL maximum (speed_kernel + dt_kernel): rho, rho u, rho v of every patch cell read",
+    "cfl": "CFL maximum (state_scan_kernel + dt_kernel): rho, rho u, rho v of every patch cell read",
 }
 
 

@@ -329,8 +329,11 @@ __device__ __forceinline__ bool same_bits(float a, float b) { return __float_as_
 //   OutRec: the tile's stored outputs, when every cell of the tile holds the
 //           same 7 values (a uniform tile, from the cache or computed);
 //   UnRec:  the tile's u^n (5 fields) and H0, when uniform over its cells and
-//           the tile lies in no absorbing band (from stage 1's uniform test).
-// A tile of stage 2 or 3 whose own input record and its eight neighbours'
+//           the tile lies in no absorbing band (from the scan at the start of
+//           the step, or from stage 1's uniform test).
+// Stage 1's own input records come from the scan (state_scan_kernel), for
+// tables of many tiles; without it stage 1 loads and tests every box.
+// A tile whose own input record and its eight neighbours'
 // (all in its patch, each reaching at least 3 cells into the halo) hold the
 // same values has a uniform halo box with those values: with a matching
 // cache entry its outputs are the entry's, and the box is not loaded.
@@ -535,7 +538,7 @@ __device__ __forceinline__ void record_out(OutRec<S>* ro, const W* wn, S pv, S t
   ro->valid = 1;
 }
 
-// The skipped tiles of a stage launch (stages 2 and 3 with skipping), taken
+// The skipped tiles of a stage launch, taken
 // by blocks that have run out of tiles to compute, eight per claim, one per
 // warp: lanes 0..12 load the tile's key from the previous stage's records;
 // the block's cache entry for the level, or else the launch's published
@@ -1179,7 +1182,7 @@ __global__ void __launch_bounds__(256, std::is_same<S, float>::value ? kStageBlo
 }
 
 // ---------------------------------------------------------------------------
-// Uniform-tile skipping, stages 2 and 3: after skip_flags_kernel, the tile
+// Uniform-tile skipping: after skip_flags_kernel, the tile
 // table is split into the tiles to compute (their descriptors and table
 // indices, in table order, so the schedule's tile orders still apply) and the
 // tiles to skip; the stage launch computes the first list, publishes its
@@ -1801,14 +1804,17 @@ __global__ void tag_block_kernel(const int* tags, int nx, int ny, int B, int buf
 // 64-bit atomicMax per block (non-negative doubles order like their bits).
 // ---------------------------------------------------------------------------
 template <typename S>
-struct SpeedArgs {
+struct ScanArgs {
   CanvasT<S> lev[kL];
+  CanvasT<S> h0[kL];
   const int4* tiles;
   const int* ntiles;
   double c;
   int ec;          // c >= 2^ec (binary exponent of c); -4096 when c is not a positive normal
   double rho_off;  // ambient density held out of the storage (0 for absolute)
   unsigned long long* smax_bits;
+  OutRec<S>* rec;    // per tile: the state, when uniform over the tile
+  UnRec<S>* rec_un;  // per tile: u^n and H0, when uniform over the tile and outside the absorbing bands
 };
 
 // max(|rho u|, |rho v|) / |rho| is max(|u|, |v|) bit for bit (a correctly
@@ -1819,12 +1825,9 @@ struct SpeedArgs {
 // compared as integers, a quotient provably below a quarter unit in the last
 // place of c (exponents alone show it) contributes c exactly, and the rest
 // divide in FP64 only when a single-precision estimate, built from the
-// doubles' exponent and leading mantissa bits, says they may hold the block's
-// maximum (FP64 division costs about nine fused multiply-adds).  The maximum
-// is the same double as dividing every cell.
-// Each block takes kSpeedTiles tiles per pass with all their loads in flight
-// together (the pass is a chain of dependent loads: descriptor, then fields).
-constexpr int kSpeedTiles = 4;
+// doubles' exponent and leading mantissa bits, says they may hold the warp's
+// maximum so far (FP64 division costs about nine fused multiply-adds).  The
+// maximum is the same double as dividing every cell.
 
 // Single-precision value of a non-negative double whose biased exponent e
 // lies in [1023 - 120, 1023 + 120]: exponent rebiased, mantissa truncated to
@@ -1833,113 +1836,167 @@ __device__ __forceinline__ float f32_of_bits(unsigned long long u, int e) {
   return __int_as_float(((e - 896) << 23) | (int)((u >> 29) & 0x7fffffu));
 }
 
-template <typename S>
-__global__ void speed_kernel(SpeedArgs<S> A) {
+__device__ __forceinline__ unsigned long long bits_of(double a) { return (unsigned long long)__double_as_longlong(a); }
+__device__ __forceinline__ unsigned bits_of(float a) { return __float_as_uint(a); }
+
+// One pass over the state at the start of a step: the CFL maximum and, with
+// records, which tiles hold one value per field, for stage 1's skipping.  A
+// warp takes a tile, two rows at a time with the next two rows' loads in
+// flight; a cell's value is compared with the tile's first by one logic
+// operation a word.  Bound by its loads.  (With a block a tile and a thread a
+// cell, the rows' values compared through shuffles and shared memory, it was
+// bound by its instructions: 233 a warp for a row, 125 us for FP64 and 99 for
+// FP32 storage on the line source's 4096 x 2048.)
+template <typename S, bool REC>  // blocks an SM, all resident
+constexpr int kScanBlocks = !REC ? 4 : (std::is_same<S, float>::value ? 3 : 2);
+template <typename S, bool REC>
+__global__ void __launch_bounds__(256, kScanBlocks<S, REC>) state_scan_kernel(
+    const __grid_constant__ ScanArgs<S> A) {
+  constexpr bool kF32S = std::is_same<S, float>::value;
+  using U = decltype(bits_of(S(0)));
   __shared__ double s_w[8];
-  __shared__ float s_e[8];
   const int n = *A.ntiles;
-  const int tx = threadIdx.x & 31, ty = threadIdx.x >> 5;
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
   double m = 0.0;
   float mf = 0.f;          // FP32 storage: the largest speed
   bool nan_seen = false;   // FP32 storage: a NaN speed (forces a tiny dt)
   bool zero_q = false;     // FP64 storage: a cell whose speed is exactly c
-  float m64est = 0.f;      // FP64 storage: the largest quotient estimate of the pass
+  float best = 0.f;        // FP64 storage: the warp's largest quotient estimate so far
   const float roff = (float)A.rho_off, cf = (float)A.c;
-  float cand_q[kSpeedTiles];
-  double av[kSpeedTiles], bv[kSpeedTiles];
+  const int step = gridDim.x * 8;
+  auto load = [&](const int4& d, int r0, S (&x)[2][8]) {
+    const int lvl = d.z & 0xff, w = (d.z >> 8) & 0xff, h = (d.z >> 16) & 0xff;
+    if (lane >= w) return;
+    const CanvasT<S>& V = A.lev[lvl];
+    const S* hb = A.h0[lvl].base;
 #pragma unroll
-  for (int u = 0; u < kSpeedTiles; ++u) cand_q[u] = -1.f;
-  for (int t0 = blockIdx.x; t0 < n; t0 += kSpeedTiles * gridDim.x) {
-    int4 td[kSpeedTiles];
+    for (int r = 0; r < 2; ++r) {
+      if (r0 + r >= h) continue;
+      const long g = (long)(d.y + r0 + r + 3) * V.pitch + (d.x + lane + 3);
+      const S* q = V.base + g;
 #pragma unroll
-    for (int u = 0; u < kSpeedTiles; ++u) {
-      const int t = t0 + u * gridDim.x;
-      td[u] = t < n ? A.tiles[t] : make_int4(0, 0, 0, 0);  // w = h = 0: no cell
-    }
-    S r[kSpeedTiles], mu[kSpeedTiles], mv[kSpeedTiles];
-    bool ok[kSpeedTiles];
+      for (int k = 0; k < 3; ++k) x[r][k] = q[k * V.fstride];
+      if constexpr (REC) {
 #pragma unroll
-    for (int u = 0; u < kSpeedTiles; ++u) {
-      const int lvl = td[u].z & 0xff, w = (td[u].z >> 8) & 0xff, h = (td[u].z >> 16) & 0xff;
-      ok[u] = tx < w && ty < h;
-      if (ok[u]) {
-        const CanvasT<S>& V = A.lev[lvl];
-        const int i = td[u].x + tx, j = td[u].y + ty;
-        r[u] = V.at(0, i, j);
-        mu[u] = V.at(1, i, j);
-        mv[u] = V.at(2, i, j);
+        for (int k = 3; k < 7; ++k) x[r][k] = q[k * V.fstride];
+        x[r][7] = hb[g];
       }
     }
+  };
+  const int4 none = make_int4(0, 0, 0, 0);  // w = h = 0: no cell
+  int t = blockIdx.x * 8 + warp;
+  int4 td = t < n ? A.tiles[t] : none, nd = t + step < n ? A.tiles[t + step] : none;
+  S buf[2][2][8];
+  load(td, 0, buf[0]);
+  for (; t < n; t += step) {
+    const int4 d2 = t + 2 * step < n ? A.tiles[t + 2 * step] : none;
+    const int w = (td.z >> 8) & 0xff, h = (td.z >> 16) & 0xff;
+    U first[8], acc = 0;
+    float est[8], top = best;
 #pragma unroll
-    for (int u = 0; u < kSpeedTiles; ++u) {
-      if (!ok[u]) continue;
-      if constexpr (std::is_same<S, float>::value) {
-        const float sf = fmaxf(fabsf(mu[u]), fabsf(mv[u])) / fabsf(roff + r[u]) + cf;
-        if (sf == sf) mf = fmaxf(mf, sf);
-        else nan_seen = true;
-      } else {
-        constexpr unsigned long long kAbs = 0x7fffffffffffffffull, kInf = 0x7ff0000000000000ull;
-        unsigned long long ua = (unsigned long long)__double_as_longlong(mu[u]) & kAbs;
-        unsigned long long uv = (unsigned long long)__double_as_longlong(mv[u]) & kAbs;
-        // fmax: a NaN operand yields the other one
-        if (ua > kInf) ua = uv;
-        else if (uv > kInf) uv = ua;
-        const unsigned long long qa = ua > uv ? ua : uv;
-        const unsigned long long qb = (unsigned long long)__double_as_longlong(r[u]) & kAbs;
-        const int ea = (int)(qa >> 52), eb = (int)(qb >> 52);
-        bool odd = true;
-        if (qb != 0 && qb <= kInf) {  // |rho| > 0, not NaN
-          // a < 2^(ea-1022) and b >= 2^(eb-1023) (b normal): the quotient is
-          // below 2^(ec-54), a quarter ulp of c, so q + c rounds to c
-          if (qa == 0 || (ea < 2047 && eb >= 1 && eb < 2047 && ea - eb <= A.ec - 55)) {
-            zero_q = true;
-            odd = false;
-          } else if (ea >= 903 && ea <= 1143 && eb >= 903 && eb <= 1143) {
-            const float qe = __fdividef(f32_of_bits(qa, ea), f32_of_bits(qb, eb));
-            if (qe > 0.f && qe < 1e30f) {
-              cand_q[u] = qe;
-              m64est = fmaxf(m64est, qe);
+    for (int q = 0; q < 4; ++q) {
+      S(&v)[2][8] = buf[q & 1];
+      if (q < 3) load(td, 2 * q + 2, buf[(q + 1) & 1]);
+      else load(nd, 0, buf[(q + 1) & 1]);
+      if constexpr (REC) {
+        if (q == 0)
+#pragma unroll
+          for (int k = 0; k < 8; ++k) first[k] = __shfl_sync(0xffffffffu, bits_of(v[0][k]), 0);
+#pragma unroll
+        for (int r = 0; r < 2; ++r)
+          if (lane < w && 2 * q + r < h)
+#pragma unroll
+            for (int k = 0; k < 8; ++k) acc |= bits_of(v[r][k]) ^ first[k];
+      }
+#pragma unroll
+      for (int r = 0; r < 2; ++r) {
+        est[2 * q + r] = -1.f;
+        if (lane >= w || 2 * q + r >= h) continue;
+        if constexpr (kF32S) {
+          const float sf = fmaxf(fabsf(v[r][1]), fabsf(v[r][2])) / fabsf(roff + v[r][0]) + cf;
+          if (sf == sf) mf = fmaxf(mf, sf);
+          else nan_seen = true;
+        } else {
+          constexpr unsigned long long kAbs = 0x7fffffffffffffffull, kInf = 0x7ff0000000000000ull;
+          unsigned long long ua = bits_of(v[r][1]) & kAbs, uv = bits_of(v[r][2]) & kAbs;
+          // fmax: a NaN operand yields the other one
+          if (ua > kInf) ua = uv;
+          else if (uv > kInf) uv = ua;
+          const unsigned long long qa = ua > uv ? ua : uv;
+          const unsigned long long qb = bits_of(v[r][0]) & kAbs;
+          const int ea = (int)(qa >> 52), eb = (int)(qb >> 52);
+          bool odd = true;
+          if (qb != 0 && qb <= kInf) {  // |rho| > 0, not NaN
+            // a < 2^(ea-1022) and b >= 2^(eb-1023) (b normal): the quotient is
+            // below 2^(ec-54), a quarter ulp of c, so q + c rounds to c
+            if (qa == 0 || (ea < 2047 && eb >= 1 && eb < 2047 && ea - eb <= A.ec - 55)) {
+              zero_q = true;
               odd = false;
+            } else if (ea >= 903 && ea <= 1143 && eb >= 903 && eb <= 1143) {
+              const float qe = __fdividef(f32_of_bits(qa, ea), f32_of_bits(qb, eb));
+              if (qe > 0.f && qe < 1e30f) {
+                est[2 * q + r] = qe;
+                top = fmaxf(top, qe);
+                odd = false;
+              }
             }
           }
+          if (odd) {
+            // outside the estimate's range: zero or subnormal density, infinite
+            // or NaN values, quotients beyond single precision
+            double x = __longlong_as_double((long long)qa) / __longlong_as_double((long long)qb);
+            if (!(x == x)) x = 1e300;  // NaN state: force a tiny dt, health check reports it
+            m = fmax(m, x + A.c);
+          }
         }
-        const double a = __longlong_as_double((long long)qa), b = __longlong_as_double((long long)qb);
-        if (odd) {
-          // outside the estimate's range: zero or subnormal density, infinite
-          // or NaN values, quotients beyond single precision
-          double q = a / b;
-          if (!(q == q)) q = 1e300;  // NaN state: force a tiny dt, health check reports it
-          m = fmax(m, q + A.c);
-        }
-        av[u] = a;
-        bv[u] = b;
       }
     }
-    if constexpr (!std::is_same<S, float>::value) {
-      // the block's largest estimate; a cell can hold the largest exact
-      // quotient only if its estimate is within the estimates' relative error
-      // (below 2^-21: two truncations to 23 mantissa bits and the approximate
-      // division; taken here as 1e-5) of that maximum: only those divide in
-      // FP64, so the maximum is the same double as dividing everywhere
-      float bm = m64est;
+    if constexpr (!kF32S) {
+      // a cell can hold the largest exact quotient only if its estimate is
+      // within the estimates' relative error (below 2^-21: two truncations
+      // to 23 mantissa bits and the approximate division; taken here as
+      // 1e-5) of the largest: only those divide in FP64 (their values read
+      // again, from the cache), so the maximum is the same double as
+      // dividing everywhere
+      if (__any_sync(0xffffffffu, top > best)) {
 #pragma unroll
-      for (int o = 16; o > 0; o >>= 1) bm = fmaxf(bm, __shfl_xor_sync(0xffffffffu, bm, o));
-      if ((threadIdx.x & 31) == 0) s_e[threadIdx.x >> 5] = bm;
-      __syncthreads();
-      bm = s_e[0];
-#pragma unroll
-      for (int w = 1; w < 8; ++w) bm = fmaxf(bm, s_e[w]);
-      __syncthreads();
-      const float thr = bm * (1.0f - 1e-5f);
-#pragma unroll
-      for (int u = 0; u < kSpeedTiles; ++u) {
-        if (cand_q[u] >= 0.f && cand_q[u] >= thr) m = fmax(m, av[u] / bv[u] + A.c);
-        cand_q[u] = -1.f;
+        for (int o = 16; o > 0; o >>= 1) top = fmaxf(top, __shfl_xor_sync(0xffffffffu, top, o));
+        best = top;
       }
-      m64est = 0.f;
+      const float thr = best * (1.0f - 1e-5f);
+      unsigned rows = 0u;
+#pragma unroll
+      for (int r = 0; r < 8; ++r)
+        if (est[r] >= 0.f && est[r] >= thr) rows |= 1u << r;
+      U la = 0, lb = 0;
+      for (; rows; rows &= rows - 1u) {
+        const CanvasT<S>& V = A.lev[td.z & 0xff];
+        const S* c = &V.at(0, td.x + lane, td.y + __ffs((int)rows) - 1);
+        const double a = fmax(fabs(c[V.fstride]), fabs(c[2 * V.fstride])), b = fabs(c[0]);
+        if (bits_of(a) == la && bits_of(b) == lb) continue;  // (a plateau divides once)
+        la = bits_of(a);
+        lb = bits_of(b);
+        m = fmax(m, a / b + A.c);
+      }
     }
+    if constexpr (REC) {
+      const bool uni = __all_sync(0xffffffffu, acc == 0 && ((td.z >> 24) & 15) == 0);  // (no absorbing side)
+      if (uni && lane < 7) {
+        U o = first[0];
+#pragma unroll
+        for (int k = 1; k < 7; ++k) o = lane == k ? first[k] : o;
+        reinterpret_cast<U*>(A.rec[t].v)[lane] = o;
+        if (lane < 6) reinterpret_cast<U*>(A.rec_un[t].v)[lane] = lane == 5 ? first[7] : o;
+      }
+      if (lane == 7) {
+        A.rec[t].valid = uni ? 1 : 0;
+        A.rec_un[t].valid = uni ? 1 : 0;
+      }
+    }
+    td = nd;
+    nd = d2;
   }
-  if constexpr (std::is_same<S, float>::value) {
+  if constexpr (kF32S) {
     m = (double)mf;
     if (nan_seen) m = fmax(m, 1e300);
   } else if (zero_q) {
@@ -1947,13 +2004,13 @@ __global__ void speed_kernel(SpeedArgs<S> A) {
   }
 #pragma unroll
   for (int o = 16; o > 0; o >>= 1) m = fmax(m, __shfl_xor_sync(0xffffffffu, m, o));
-  if ((threadIdx.x & 31) == 0) s_w[threadIdx.x >> 5] = m;
+  if (lane == 0) s_w[warp] = m;
   __syncthreads();
   if (threadIdx.x < 32) {
-    m = threadIdx.x < (blockDim.x >> 5) ? s_w[threadIdx.x] : 0.0;
+    m = lane < 8 ? s_w[lane] : 0.0;
 #pragma unroll
     for (int o = 16; o > 0; o >>= 1) m = fmax(m, __shfl_xor_sync(0xffffffffu, m, o));
-    if (threadIdx.x == 0) atomicMax(A.smax_bits, (unsigned long long)__double_as_longlong(m));
+    if (lane == 0) atomicMax(A.smax_bits, (unsigned long long)__double_as_longlong(m));
   }
 }
 
@@ -2352,10 +2409,11 @@ struct Engine {
   int max_blocks_per_sm = 1;
   int sched_bps = 0;  // 0: max_blocks_per_sm
   int sched_chunk = 1;
-  // uniform-tile skipping in stages 2 and 3 (with reuse): per tile the
+  // uniform-tile skipping (with reuse): per tile the
   // neighbour stride (tiles per row of its patch, 0 when a neighbour lies
   // outside the patch), this step's records and the skip flags
   int skip = 1;
+  bool many_tiles = false;  // stage 1 skips too (rebuild_tables)
   DevArray<int> d_nbr;
   std::vector<int> h_nbr;
   DevArray<unsigned char> d_rec_o1, d_rec_o2, d_rec_un, d_skip;
@@ -2736,6 +2794,21 @@ static int rebuild_tables(Engine* E) {
     grew |= E->d_bcnt.ensure((E->d_skip.cap + kFlagThreads - 1) / kFlagThreads);
   }
   if (grew) E->graph_valid = false;
+  // A table whose tiles repay stage 1's skipping: uniform tiles are the base
+  // level's (finer levels lie where the waves are).  On the 33,000 base tiles of
+  // the line source's 4096 x 2048, most of them uniform, a step takes 3.56 ms
+  // without and 3.31 with it (FP64), 0.744 and 0.638 (FP32 storage): 8 and 3 ns
+  // a tile, against 28 and 15 us for the records, flags, lists and second
+  // launch (the Mach shock, 2,048 base and 7,680 fine tiles, few of them
+  // uniform, in FP64: 9.560 and 9.587 ms).  Hence on from 16 base tiles a block
+  // of a full grid (4,864 and 9,728), off below half of that: a captured step
+  // does not change with every new table.
+  {
+    const int most = 16 * E->nsm * E->max_blocks_per_sm;
+    const bool many = nl > 0 && E->tile_cnt[0] >= (E->many_tiles ? most / 2 : most);
+    if (many != E->many_tiles) E->graph_valid = false;
+    E->many_tiles = many;
+  }
   if (!E->d_nbr.p || !E->d_skip.p || !E->d_rec_o1.p || !E->d_rec_o2.p || !E->d_rec_un.p || !E->d_full_td.p ||
       !E->d_left_td.p || !E->d_full_gti.p || !E->d_skip_gti.p || !E->d_left_gti.p || !E->d_bcnt.p) {
     E->tables_on_device = false;
@@ -2819,6 +2892,12 @@ static EosConst64 eos_const64(const enl_engine_config& c) {
 static bool skip_on(const Engine* E) {
   return E->skip && !E->cfg.dense && E->cfg.c_lr == 0.0 && !E->samrai_order && E->d_skipcnt && E->d_gcache;
 }
+
+// Stage 1 skips too where the CFL pass reads the state anyway (adaptive dt)
+// and the table is large (many_tiles).  With a fixed dt the pass over the
+// state would have to be paid for as well: 24 pulses, FP32 storage, 0.800 ms a
+// step without and 0.841 with; 64 in FP64, 18.118 and 18.120.
+static bool skip_first_on(const Engine* E) { return skip_on(E) && E->adaptive && E->many_tiles; }
 
 static StageArgs stage_args(Engine* E, int stage, double dt, int level = -1) {
   StageArgs A;
@@ -2913,14 +2992,13 @@ static StageArgs stage_args(Engine* E, int stage, double dt, int level = -1) {
   A.feat_eps_p = (float)(A.P[0].sensor_eps * (c.c * c.c) * (c.c * c.c));
   A.feat_inv_sqrt_eps = (float)(1.0 / sqrt(A.P[0].sensor_eps));
   if (skip_on(E)) {
-    // stage 1 records its outputs and u^n / H0, stage 2 its outputs; stages
-    // 2 and 3 run over the list of tiles to compute (skip_stage_t) and
-    // publish their uniform results for the skipped ones
-    if (stage == 0) {
-      A.rec_out = E->d_rec_o1.p;
+    // stages 1 and 2 record their outputs, and stage 1 u^n / H0 where the
+    // scan has not; stages that skip run over the list of tiles to compute
+    // (skip_stage_t) and publish their uniform results for the skipped ones
+    A.rec_out = stage == 0 ? E->d_rec_o1.p : (stage == 1 ? E->d_rec_o2.p : nullptr);
+    if (stage == 0 && !skip_first_on(E)) {
       A.rec_un_out = E->d_rec_un.p;
     } else {
-      A.rec_out = stage == 1 ? E->d_rec_o2.p : nullptr;
       A.tiles = E->d_full_td.p;
       A.gti = E->d_full_gti.p;
       A.ntiles = E->d_skipcnt;
@@ -3144,10 +3222,13 @@ static double finest_dx(Engine* E) {
 }
 
 template <typename S>
-static void speed_t(Engine* E) {
-  SpeedArgs<S> A;
+static void scan_t(Engine* E, bool records) {
+  ScanArgs<S> A;
   memset(&A, 0, sizeof(A));
-  for (int l = 0; l < E->cfg.nlevels; ++l) A.lev[l] = E->lev[l].view<S>(0);
+  for (int l = 0; l < E->cfg.nlevels; ++l) {
+    A.lev[l] = E->lev[l].view<S>(0);
+    A.h0[l] = E->lev[l].view<S>(3);
+  }
   A.tiles = E->d_tiles.p;
   A.ntiles = E->d_meta + M_NTILES;
   A.c = E->cfg.c;
@@ -3155,18 +3236,26 @@ static void speed_t(Engine* E) {
   A.ec = (std::isnormal(A.c) && A.c > 0.0) ? (std::frexp(A.c, &ec), ec - 1) : -4096;
   A.rho_off = E->off[0];
   A.smax_bits = E->d_smax;
-  speed_kernel<S><<<E->nsm * 8, 256, 0, stream()>>>(A);
+  if (records) {
+    A.rec = reinterpret_cast<OutRec<S>*>(E->d_rec_o2.p);  // (stage 2 writes its outputs there later)
+    A.rec_un = reinterpret_cast<UnRec<S>*>(E->d_rec_un.p);
+  }
+  if (records) state_scan_kernel<S, true><<<E->nsm * kScanBlocks<S, true>, 256, 0, stream()>>>(A);
+  else state_scan_kernel<S, false><<<E->nsm * kScanBlocks<S, false>, 256, 0, stream()>>>(A);
 }
 
-static void adaptive_dt(Engine* E, double dt_max) {
+// The pass over the state at the start of a step, and the step's dt from it.
+static void scan_state(Engine* E, double dt_max, bool records) {
   if (!E->adaptive) return;
-  // reads rho, rho u, rho v of every patch cell
+  // rho, rho u, rho v of every patch cell (uniform tiles' other fields, read
+  // for stage 1's skipping, are not counted)
   long long cells = 0;
   for (int l = 0; l < E->cfg.nlevels; ++l) cells += E->n_cells[l];
   const int q = kt_begin(E, 3, 3.0 * (E->f32s ? 4 : 8) * cells);
-  if (E->f32s) speed_t<float>(E);
-  else speed_t<double>(E);
-  dt_kernel<<<1, 1, 0, stream()>>>(E->d_smax, E->d_dt, E->d_dt + 1, reinterpret_cast<float*>(E->d_dt + 2), E->cfl * finest_dx(E), dt_max);
+  if (E->f32s) scan_t<float>(E, records);
+  else scan_t<double>(E, records);
+  dt_kernel<<<1, 1, 0, stream()>>>(E->d_smax, E->d_dt, E->d_dt + 1, reinterpret_cast<float*>(E->d_dt + 2),
+                                   E->cfl * finest_dx(E), dt_max);
   kt_end(E, q);
 }
 
@@ -3202,8 +3291,8 @@ static void record_mics(Engine* E) {
   else mics_t<double>(E);
 }
 
-// RK stage `stage` (1 or 2) with skipping: flags and lists from the previous
-// stage's records, the launch over the tiles to compute (its blocks then
+// RK stage `stage` with skipping: flags and lists from the records of its
+// input (stage 0: the scan's, in stage 1's output records' place), the launch over the tiles to compute (its blocks then
 // store the skipped tiles, skip_phase), and a launch over the skipped tiles
 // without a cached or published result (usually none).
 template <typename S>
@@ -3248,7 +3337,7 @@ static int step_fused(Engine* E, double dt) {
   cudaStream_t s = stream();
   cudaMemsetAsync(E->d_counters, 0, 3 * (1 + kL) * sizeof(int), s);
   cudaMemsetAsync(E->d_counters64, 0, 3 * (1 + kL) * sizeof(unsigned long long), s);
-  adaptive_dt(E, dt);
+  scan_state(E, dt, skip_first_on(E));
   StageFn fn = pick_stage(E->cfg.precision, E->cfg.variant);
   for (int st = 0; st < 3; ++st) {
     int in = st == 0 ? 0 : st;
@@ -3280,7 +3369,7 @@ static int step_fused(Engine* E, double dt) {
     StageArgs A = stage_args(E, st, dt);
     void* args[] = {&A};
     if (E->profile) cudaEventRecord(E->pev[2 * st], s);
-    if (st > 0 && skip_on(E)) {
+    if (st > 0 ? skip_on(E) : skip_first_on(E)) {
       if (E->f32s) skip_stage_t<float>(E, st, fn, A);
       else skip_stage_t<double>(E, st, fn, A);
     } else {
@@ -3312,7 +3401,7 @@ static int step_plain(Engine* E, double dt) {
   cudaStream_t s = stream();
   const auto& c = E->cfg;
   const int nl = c.nlevels;
-  adaptive_dt(E, dt);
+  scan_state(E, dt, false);
   // copy current -> scratch (patch interiors)
   for (int l = 0; l < nl; ++l)
     if (E->tile_cnt[l])
@@ -3858,7 +3947,8 @@ int enl_engine_launches_per_step(void* e, int plain) {
     // interpolation below level 1)
     const int refresh = E->samrai_order ? (nl - 1) + (nl > 2 ? nl - 2 : 0) : 0;
     return 3 * (bands + (nl - 1) + (E->samrai_order ? nl : 1) + refresh) + (nl - 1) + dt +
-           (skip_on(E) ? 6 : 0);  // stages 2 and 3: flags, lists, second launch
+           // skipping stages: flags, lists, second launch
+           (skip_on(E) ? 6 : 0) + (skip_first_on(E) ? 3 : 0);
   }
   const int absorbs = any_absorb(E) ? 1 : 0;
   int npatch = 0, copies = 0;
@@ -4363,7 +4453,7 @@ int enl_engine_mic_records(void* e, void* host, long long max, long long* n, lon
 //   [1] tile order: 0 finest level first, 1 level 0 first, 2 the two ends
 //       of the tile table alternately, 3 two streams (each SM's first block
 //       from the finest end, its second from level 0),
-//   [2] uniform-tile reuse: 2 on, with stages 2 and 3 skipping the halo box
+//   [2] uniform-tile reuse: 2 on, with the stages skipping the halo box
 //       of tiles this step's records prove uniform; 1 on, every box loaded
 //       and tested; 0 every tile computed cell by cell (results identical
 //       in all three),

@@ -1,7 +1,7 @@
 // Stable time step of one patch without any device allocation.
 //
 // enl_cfl_dt_static computes, for one patch in SAMRAI CellData layout, the
-// same time step as the engine's device CFL reduction (speed_kernel +
+// same time step as the engine's device CFL reduction (state_scan_kernel +
 // dt_kernel in enl_engine.cu):
 //   dt = min(dt_max, cfl * dx_min / max over the interior of max(|u|,|v|) + c)
 // The engine keeps its reduction word in memory it allocates with
