@@ -1397,13 +1397,60 @@ __device__ __forceinline__ void refine_weights(int I, int r, int& ic, S& f) {
   f = xc - fl;
 }
 
+// The 7 fields of fine cell (I, J) from the coarser canvas, every coarse load
+// issued before the first use (a store of the caller could alias a later load,
+// so the compiler would not move those loads above it).  FP64 at ratio 2: the
+// cell lies a quarter of a coarse cell from the centre of its own, so the
+// weights are 9, 3, 3 and 1 sixteenths: four FP64 operations a field where the
+// weights and three interpolations took six and the cell's weights thirty, on
+// a pipe of 1/64 of the FP32 rate (interpolation of the line source's two finer
+// levels, 4096 x 2048: 14.5 + 26 us before, LINEINTERP now).  Equal coarse values give
+// that value exactly, as before: c/16, 3/8 c + c/16 and 9/16 c + rnd(7/16 c),
+// whose error stays below half a unit in c's last place.
+template <typename S>
+__device__ __forceinline__ void refined(const CanvasT<S>& C, int ratio, int I, int J, S v[kNF]) {
+  if constexpr (std::is_same<S, double>::value) {
+    if (ratio == 2) {
+      const S* c = &C.at(0, I >> 1, J >> 1);
+      const long dx = (I & 1) ? 1 : -1, dy = (J & 1) ? C.pitch : -C.pitch;
+      S a[kNF], b[kNF], d[kNF], e[kNF];
+#pragma unroll
+      for (int k = 0; k < kNF; ++k, c += C.fstride) {
+        a[k] = c[0];
+        b[k] = c[dx];
+        d[k] = c[dy];
+        e[k] = c[dx + dy];
+      }
+#pragma unroll
+      for (int k = 0; k < kNF; ++k) v[k] = fma(0.5625, a[k], fma(0.1875, b[k] + d[k], 0.0625 * e[k]));
+      return;
+    }
+  }
+  int jc, ic;
+  S fy, fx;
+  refine_weights(J, ratio, jc, fy);
+  refine_weights(I, ratio, ic, fx);
+  S c00[kNF], c10[kNF], c01[kNF], c11[kNF];
+#pragma unroll
+  for (int k = 0; k < kNF; ++k) {
+    c00[k] = C.at(k, ic, jc);
+    c10[k] = C.at(k, ic + 1, jc);
+    c01[k] = C.at(k, ic, jc + 1);
+    c11[k] = C.at(k, ic + 1, jc + 1);
+  }
+#pragma unroll
+  for (int k = 0; k < kNF; ++k) {
+    S lo_ = ((S)1 - fx) * c00[k] + fx * c10[k];
+    S hi_ = ((S)1 - fx) * c01[k] + fx * c11[k];
+    v[k] = ((S)1 - fy) * lo_ + fy * hi_;
+  }
+}
+
 // One warp per halo chunk (a row run of at most 32 cells of the level's halo,
 // the tables split longer runs), one lane per cell: a lane finds its cell
 // without a search and has its 4 x nfields loads in flight together.
 // Consecutive chunks go to different blocks, so a halo of a few hundred
-// chunks still spreads over every SM.  All 4 x 7 coarse loads of a lane are
-// issued before its first store (a store could alias a later load, so the
-// compiler would not move those loads above it).
+// chunks still spreads over every SM.
 template <typename S>
 __global__ void interp_kernel(CanvasT<S> F, CanvasT<S> C, int ratio, const int4* segs, const int* meta, int moff,
                               int mcnt) {
@@ -1413,32 +1460,27 @@ __global__ void interp_kernel(CanvasT<S> F, CanvasT<S> C, int ratio, const int4*
     const int4 sg = segs[off + q];
     const int J = sg.x, I = sg.y + lane;
     if (I > sg.z) continue;
-    int jc, ic;
-    S fy, fx;
-    refine_weights(J, ratio, jc, fy);
-    refine_weights(I, ratio, ic, fx);
-    S c00[kNF], c10[kNF], c01[kNF], c11[kNF];
+    S v[kNF];
+    refined(C, ratio, I, J, v);
 #pragma unroll
-    for (int k = 0; k < kNF; ++k) {
-      c00[k] = C.at(k, ic, jc);
-      c10[k] = C.at(k, ic + 1, jc);
-      c01[k] = C.at(k, ic, jc + 1);
-      c11[k] = C.at(k, ic + 1, jc + 1);
-    }
-#pragma unroll
-    for (int k = 0; k < kNF; ++k) {
-      S lo_ = ((S)1 - fx) * c00[k] + fx * c10[k];
-      S hi_ = ((S)1 - fx) * c01[k] + fx * c11[k];
-      F.at(k, I, J) = ((S)1 - fy) * lo_ + fy * hi_;
-    }
+    for (int k = 0; k < kNF; ++k) F.at(k, I, J) = v[k];
   }
 }
+
+// s/4, exactly s * 0.25, without the FP64 pipe where the exponent allows.
+__device__ __forceinline__ double quarter(double s) {
+  const int hi = __double2hiint(s), e = (hi >> 20) & 0x7ff;
+  return e > 2 && e < 2047 ? __hiloint2double(hi - (2 << 20), __double2loint(s)) : s * 0.25;
+}
+__device__ __forceinline__ float quarter(float s) { return s * 0.25f; }
 
 // Generic tile-list kernels: one block of 256 threads per 32x8 tile.
 // Coarsening: coarse cell = mean of its ratio x ratio fine cells (7 fields).
 // A block takes one field of one tile, so the few tiles a fine level covers
 // still spread over every SM; at ratio 2 a thread's four loads are issued
-// together (the sum keeps the row-major order of the general loop).
+// together (the sum keeps the row-major order of the general loop), and FP64
+// takes three operations a cell instead of five (the Mach shock's 7,680 fine
+// tiles: SHOCKCOARSEN).
 template <typename S>
 __global__ void coarsen_kernel(CanvasT<S> C, CanvasT<S> F, int ratio, const int4* tiles, const int* meta, int moff,
                                int mcnt) {
@@ -1451,19 +1493,16 @@ __global__ void coarsen_kernel(CanvasT<S> C, CanvasT<S> F, int ratio, const int4
     const int w = (td.z >> 8) & 0xff, h = (td.z >> 16) & 0xff;
     if (tx >= w || ty >= h) continue;
     const int I = td.x + tx, J = td.y + ty;
-    S s = 0;
     if (ratio == 2) {
       const S f00 = F.at(k, 2 * I, 2 * J), f10 = F.at(k, 2 * I + 1, 2 * J);
       const S f01 = F.at(k, 2 * I, 2 * J + 1), f11 = F.at(k, 2 * I + 1, 2 * J + 1);
-      s += f00;
-      s += f10;
-      s += f01;
-      s += f11;
+      C.at(k, I, J) = quarter(((f00 + f10) + f01) + f11);
     } else {
+      S s = 0;
       for (int b = 0; b < ratio; ++b)
         for (int a = 0; a < ratio; ++a) s += F.at(k, I * ratio + a, J * ratio + b);
+      C.at(k, I, J) = s * inv;
     }
-    C.at(k, I, J) = s * inv;
   }
 }
 
@@ -1479,27 +1518,21 @@ __global__ void copy_tiles_kernel(CanvasT<S> dst, CanvasT<S> src, const int4* ti
   }
 }
 
-// Bilinear fill of whole boxes (new fine data after a regrid).
+// Bilinear fill of whole boxes (new fine data after a regrid): blockIdx.y picks
+// the box (ilo, ihi, jlo, jhi) of `boxes`; the blocks along x share its cells
+// (fewer than 2^31: a cell of a level takes 176 or 88 bytes).
 template <typename S>
-// blockIdx.y picks the box (ilo, ihi, jlo, jhi) of `boxes`; the blocks along
-// x share its cells.
 __global__ void refine_box_kernel(CanvasT<S> F, CanvasT<S> C, int ratio, const int4* boxes, int nbox) {
   for (int q = blockIdx.y; q < nbox; q += gridDim.y) {
-  const int4 bx = boxes[q];
-  const int ilo = bx.x, jlo = bx.z, w = bx.y - bx.x + 1, h = bx.w - bx.z + 1;
-  long n = (long)w * h;
-  for (long t = blockIdx.x * (long)blockDim.x + threadIdx.x; t < n; t += (long)gridDim.x * blockDim.x) {
-    int I = ilo + (int)(t % w), J = jlo + (int)(t / w);
-    int ic, jc;
-    S fx, fy;
-    refine_weights(I, ratio, ic, fx);
-    refine_weights(J, ratio, jc, fy);
-    for (int k = 0; k < kNF; ++k) {
-      S lo = ((S)1 - fx) * C.at(k, ic, jc) + fx * C.at(k, ic + 1, jc);
-      S hi = ((S)1 - fx) * C.at(k, ic, jc + 1) + fx * C.at(k, ic + 1, jc + 1);
-      F.at(k, I, J) = ((S)1 - fy) * lo + fy * hi;
+    const int4 bx = boxes[q];
+    const unsigned w = bx.y - bx.x + 1, n = w * (unsigned)(bx.w - bx.z + 1);
+    for (unsigned t = blockIdx.x * blockDim.x + threadIdx.x; t < n; t += gridDim.x * blockDim.x) {
+      const int I = bx.x + (int)(t % w), J = bx.z + (int)(t / w);
+      S v[kNF];
+      refined(C, ratio, I, J, v);
+#pragma unroll
+      for (int k = 0; k < kNF; ++k) F.at(k, I, J) = v[k];
     }
-  }
   }
 }
 
