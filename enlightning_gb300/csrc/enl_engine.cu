@@ -1404,7 +1404,7 @@ __device__ __forceinline__ void refine_weights(int I, int r, int& ic, S& f) {
 // weights are 9, 3, 3 and 1 sixteenths: four FP64 operations a field where the
 // weights and three interpolations took six and the cell's weights thirty, on
 // a pipe of 1/64 of the FP32 rate (interpolation of the line source's two finer
-// levels, 4096 x 2048: 14.5 + 26 us before, LINEINTERP now).  Equal coarse values give
+// levels, 4096 x 2048: 14.5 + 26 us before, 10.3 + 16.5 now).  Equal coarse values give
 // that value exactly, as before: c/16, 3/8 c + c/16 and 9/16 c + rnd(7/16 c),
 // whose error stays below half a unit in c's last place.
 template <typename S>
@@ -1479,8 +1479,8 @@ __device__ __forceinline__ float quarter(float s) { return s * 0.25f; }
 // A block takes one field of one tile, so the few tiles a fine level covers
 // still spread over every SM; at ratio 2 a thread's four loads are issued
 // together (the sum keeps the row-major order of the general loop), and FP64
-// takes three operations a cell instead of five (the Mach shock's 7,680 fine
-// tiles: SHOCKCOARSEN).
+// takes three operations a cell instead of five (line source, two levels: 14.3
+// + 8.1 us before, 12.1 + 7.2 now).
 template <typename S>
 __global__ void coarsen_kernel(CanvasT<S> C, CanvasT<S> F, int ratio, const int4* tiles, const int* meta, int moff,
                                int mcnt) {
