@@ -1542,6 +1542,7 @@ __global__ void refine_box_kernel(CanvasT<S> F, CanvasT<S> C, int ratio, const i
 // on this part and the fast engine's tags need no bit-exactness); 0.9999f is
 // the reference's REAL*4 literal itself.
 __device__ __forceinline__ bool ratio_below_f(float fm, float f0, float fp, float ep) {
+  if (same_bits(fm, f0) && same_bits(fp, f0)) return false;  // as tag_line64
   const float t1 = f0 - fm, t2 = fp - f0;
   const float num = fmaf(2.0f, fabsf(t1 * t2), ep);
   const float den = fmaf(t1, t1, fmaf(t2, t2, ep));
@@ -1566,10 +1567,12 @@ __global__ void tag_tiles_kernel(int* tags, CanvasT<S> W, CanvasT<S> H, const in
     bool tg;
     if constexpr (std::is_same<S, float>::value) {
       const float e0 = (float)ep0, e1 = (float)ep1;
-      tg = ratio_below_f(H.at(0, i - 1, j), H.at(0, i, j), H.at(0, i + 1, j), e0) ||
-           ratio_below_f(H.at(0, i, j - 1), H.at(0, i, j), H.at(0, i, j + 1), e0) ||
-           ratio_below_f(W.at(0, i - 1, j), W.at(0, i, j), W.at(0, i + 1, j), e1) ||
-           ratio_below_f(W.at(0, i, j - 1), W.at(0, i, j), W.at(0, i, j + 1), e1);
+      const float* hp = &H.at(0, i, j);
+      const float* rp = &W.at(0, i, j);
+      const float h[5] = {hp[0], hp[-1], hp[1], hp[-H.pitch], hp[H.pitch]};
+      const float r[5] = {rp[0], rp[-1], rp[1], rp[-W.pitch], rp[W.pitch]};
+      tg = ratio_below_f(h[1], h[0], h[2], e0) || ratio_below_f(h[3], h[0], h[4], e0) ||
+           ratio_below_f(r[1], r[0], r[2], e1) || ratio_below_f(r[3], r[0], r[4], e1);
     } else {
       tg = tag_cell64(&H.at(0, i, j), &W.at(0, i, j), W.pitch, ep0, ep0f, ep1, ep1f);
     }
@@ -1759,11 +1762,12 @@ __device__ __forceinline__ void bbox_merge(int* bbox, unsigned char any, int bx,
     const int x1 = __reduce_max_sync(0xffffffffu, any ? bx : -1);
     const int y0 = __reduce_min_sync(0xffffffffu, any ? by : 0x7fffffff);
     const int y1 = __reduce_max_sync(0xffffffffu, any ? by : -1);
-    if ((threadIdx.x & 31) == 0) {
-      atomicMin(&bbox[0], x0);
-      atomicMax(&bbox[1], x1);
-      atomicMin(&bbox[2], y0);
-      atomicMax(&bbox[3], y1);
+    if ((threadIdx.x & 31) == 0) {  // (most warps lie inside the box already)
+      const volatile int* now = bbox;
+      if (x0 < now[0]) atomicMin(&bbox[0], x0);
+      if (x1 > now[1]) atomicMax(&bbox[1], x1);
+      if (y0 < now[2]) atomicMin(&bbox[2], y0);
+      if (y1 > now[3]) atomicMax(&bbox[3], y1);
     }
   }
 }
@@ -1776,15 +1780,15 @@ __device__ __forceinline__ void bbox_merge(int* bbox, unsigned char any, int bx,
 __global__ void tag_dilate_kernel(const unsigned long long* __restrict__ mask, int nbx, int nby,
                                   unsigned long long rm0, unsigned long long rm2, unsigned long long cm0,
                                   unsigned long long cm2, unsigned char* map, int* bbox) {
-  const long n = (long)nbx * nby;
-  const long stride = (long)gridDim.x * blockDim.x;
-  for (long t0 = blockIdx.x * (long)blockDim.x; t0 < n; t0 += stride) {  // trip count uniform per warp
-    const long t = t0 + threadIdx.x;
+  const unsigned n = (unsigned)nbx * (unsigned)nby;  // (fewer blocks than cells: below 2^31)
+  const unsigned stride = gridDim.x * blockDim.x;
+  for (unsigned t0 = blockIdx.x * blockDim.x; t0 < n; t0 += stride) {  // trip count uniform per warp
+    const unsigned t = t0 + threadIdx.x;
     unsigned char any = 0;
     int bx = 0, by = 0;
     if (t < n) {
-      bx = (int)(t % nbx);
-      by = (int)(t / nbx);
+      bx = (int)(t % (unsigned)nbx);
+      by = (int)(t / (unsigned)nbx);
       const unsigned long long all = ~0ull;
       const unsigned long long rm[3] = {rm0, all, rm2}, cm[3] = {cm0, all, cm2};
       unsigned long long hit = 0;
