@@ -1467,6 +1467,37 @@ __global__ void interp_kernel(CanvasT<S> F, CanvasT<S> C, int ratio, const int4*
   }
 }
 
+// Coarse index of the lower of the two coarse cells a fine cell interpolates
+// from: floor((I + 1/2)/r - 1/2), as refine_weights.
+__device__ __forceinline__ int coarse_lo(int I, int r) {
+  const int n = 2 * I + 1 - r, d = 2 * r;
+  return n >= 0 ? n / d : -((-n + d - 1) / d);
+}
+
+// Distinct coarse cells under the 2 x 2 stencils of a level's halo chunks (the
+// interpolation's reads, for the kernel-class profile): a bit per coarse cell,
+// ghosts at -1 and nx included, in rows of `words`; who sets a bit counts it.  A
+// warp takes a chunk, a lane one word of one of its two coarse rows.  (Sorting
+// the chunks' intervals on the host was 160 us of every rebuild of the tables,
+// a quarter of the line source's regrid, profiled or not.)
+__global__ void halo_coarse_kernel(const int4* segs, int cnt, int ratio, int words, unsigned* bits,
+                                   unsigned long long* total) {
+  const int lane = threadIdx.x & 31;
+  int n = 0;
+  for (int q = (blockIdx.x * blockDim.x + threadIdx.x) >> 5; q < cnt; q += (gridDim.x * blockDim.x) >> 5) {
+    const int4 sg = segs[q];
+    const int row = coarse_lo(sg.x, ratio) + 1 + (lane & 1);
+    const int a = coarse_lo(sg.y, ratio) + 1, b = coarse_lo(sg.z, ratio) + 2;
+    const int wd = (a >> 5) + (lane >> 1);
+    if (wd > (b >> 5)) continue;
+    const int lo = max(a, 32 * wd) & 31, hi = min(b, 32 * wd + 31) & 31;
+    const unsigned m = (0xffffffffu >> (31 - hi)) & (0xffffffffu << lo);
+    n += __popc(m & ~atomicOr(&bits[(long)row * words + wd], m));
+  }
+  n = __reduce_add_sync(0xffffffffu, n);
+  if (lane == 0 && n) atomicAdd(total, (unsigned long long)n);
+}
+
 // s/4, exactly s * 0.25, without the FP64 pipe where the exponent allows.
 __device__ __forceinline__ double quarter(double s) {
   const int hi = __double2hiint(s), e = (hi >> 20) & 0x7ff;
@@ -2637,37 +2668,8 @@ static void level_neighbours(const std::vector<int4>& tiles, const std::vector<i
   }
 }
 
-// Coarse index of the lower of the two coarse cells a fine cell
-// interpolates from: floor((I + 1/2)/r - 1/2), as refine_weights.
-static int coarse_lo(int I, int r) {
-  const int n = 2 * I + 1 - r, d = 2 * r;
-  return n >= 0 ? n / d : -((-n + d - 1) / d);
-}
-
 // Sizes the profile mode's byte counts use, for level l of the tables.
 static void level_counts(Engine* E, int l) {
-  const int r = E->cfg.ratio;
-  long long hc = 0;
-  if (l > 0) {
-    // distinct coarse cells under the halo's 2 x 2 stencils: row intervals
-    // per coarse row, merged
-    std::vector<int3> iv;
-    const int off = E->h_meta[M_HALO_OFF + l], cnt = E->h_meta[M_HALO_CNT + l];
-    iv.reserve(2 * (size_t)cnt);
-    for (int q = off; q < off + cnt; ++q) {
-      const int4 sg = E->h_halo[q];
-      const int jc = coarse_lo(sg.x, r), a = coarse_lo(sg.y, r), b = coarse_lo(sg.z, r) + 1;
-      iv.push_back(make_int3(jc, a, b));
-      iv.push_back(make_int3(jc + 1, a, b));
-    }
-    std::sort(iv.begin(), iv.end(), [](const int3& u, const int3& v) { return u.x != v.x ? u.x < v.x : u.y < v.y; });
-    for (size_t k = 0; k < iv.size();) {
-      int row = iv[k].x, lo = iv[k].y, hi = iv[k].z;
-      for (++k; k < iv.size() && iv[k].x == row && iv[k].y <= hi + 1; ++k) hi = std::max(hi, iv[k].z);
-      hc += hi - lo + 1;
-    }
-  }
-  E->n_halo_coarse[l] = hc;
   long long cc = 0;
   for (int q = E->h_meta[M_CT_OFF + l]; q < E->h_meta[M_CT_OFF + l] + E->h_meta[M_CT_CNT + l]; ++q)
     cc += (long long)((E->h_ctiles[q].z >> 8) & 0xff) * ((E->h_ctiles[q].z >> 16) & 0xff);
@@ -2700,6 +2702,31 @@ static long long band_cells(int nx, int ny, int sides) {
 static bool any_absorb(const Engine* E);
 static AbsorbTables absorb_tables(const Engine* E);
 static AbsorbTables absorb_tables_host(const Engine* E);
+
+// E->n_halo_coarse of every level, from the tables on the device.
+static void count_halo_coarse(Engine* E) {
+  cudaStream_t s = stream();
+  for (int l = 1; l < E->cfg.nlevels; ++l) {
+    const Level& C = E->lev[l - 1];
+    const int words = (C.nx + 2 + 31) / 32;
+    const size_t nb = (size_t)words * (C.ny + 2) * sizeof(unsigned);
+    unsigned char* d = nullptr;
+    unsigned long long n = 0;
+    E->n_halo_coarse[l] = 0;
+    if (E->h_meta[M_HALO_CNT + l] == 0 || cudaMalloc(&d, nb + 8) != cudaSuccess) {
+      cudaGetLastError();  // (a count of 0: the profile's bytes lack it)
+      continue;
+    }
+    cudaMemsetAsync(d, 0, nb + 8, s);  // the count first, then the bits
+    halo_coarse_kernel<<<E->nsm, 256, 0, s>>>(E->d_halo.p + E->h_meta[M_HALO_OFF + l], E->h_meta[M_HALO_CNT + l],
+                                              E->cfg.ratio, words, reinterpret_cast<unsigned*>(d + 8),
+                                              reinterpret_cast<unsigned long long*>(d));
+    cudaMemcpyAsync(&n, d, sizeof(n), cudaMemcpyDeviceToHost, s);
+    cudaStreamSynchronize(s);
+    cudaFree(d);
+    E->n_halo_coarse[l] = (long long)n;
+  }
+}
 
 static int rebuild_tables(Engine* E) {
   const int nl = E->cfg.nlevels;
@@ -2901,6 +2928,7 @@ static int rebuild_tables(Engine* E) {
   put(E->d_meta, E->h_meta, b_meta);
   cudaEventRecord(E->stage_ev, s);
   E->tables_on_device = true;
+  if (E->profile >= 2) count_halo_coarse(E);
   return check_launch("engine tables");
 }
 
@@ -4928,7 +4956,9 @@ int enl_engine_profile(void* e, int on, double* ms_total, long long* launches, l
   }
   if (on && !E->pev[0])
     for (int q = 0; q < 6; ++q) cudaEventCreate(&E->pev[q]);
+  const bool was = E->profile >= 2;
   E->profile = on <= 0 ? 0 : on >= 2 ? 2 : 1;
+  if (E->profile >= 2 && !was && E->tables_on_device) count_halo_coarse(E);
   return check_launch("engine profile");
 }
 
