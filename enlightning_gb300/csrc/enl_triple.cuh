@@ -7,10 +7,11 @@
 // the nonlinear part runs on the FP32 pipe with numbers of three floats
 // (value = h + m + l, each word about 2^-23 of the one before, relative error
 // of one operation below 2^-60).  One flux difference (four reconstructions)
-// takes about 26 clocks of an SM; in FP64 it was about 155 instructions of the
+// took about 26 clocks of an SM; in FP64 it was about 155 instructions of the
 // FP64 pipe, 78 clocks.  On the Mach shock (1024x512, two levels, WENO nearly
 // everywhere) an FP64 step went from 29.8 to 11.3 ms, on the three-level line
-// source with its host exchange from 9.2 to 5.0 ms.
+// source with its host exchange from 9.2 to 5.0 ms.  (Since then t3_grid has
+// taken a tenth off its operations.)
 //
 // Accuracy, against 128-bit arithmetic on 200,000 random stencils each (error
 // over the stencil's largest split flux, RMS): smooth waves 2.0e-18 (FP64
@@ -133,6 +134,37 @@ __device__ __forceinline__ T3 t3_mul_f(T3 a, f2 c) {
   return T3{p, s, f2_fma(c, a.l, f2_add(f, r))};
 }
 
+// Sums of the differences with small whole coefficients, on a common grid: the
+// words of a value below 2 in magnitude are put on multiples of 2^-19 and
+// 2^-40 and a rest (12 operations), where values of the same scale add word
+// by word, exactly in the first two (up to 8 of them: 2^24 steps of the grid),
+// three operations a sum; what is then squared is made three words of
+// decreasing size again (nine).  Against t3_add, 22 operations, 15 times a flux
+// difference, it leaves 195 of 330 (of 1331 in all): the Mach shock's step
+// 9.55 -> 9.00 ms, the line source's 3.26 -> 3.11, a small two-level run's 0.364
+// -> 0.344.  The grid ends near 2^-63 of the largest
+// difference: a small value next to a large one loses relative accuracy, but
+// the weights it forms differ from 0 and 1 only where the differences they
+// multiply are as small (errors on 200,000 random stencils as in the heading;
+// noise of 1e-11 beside a jump 2.0e-20 of the flux instead of 1.3e-21).
+__device__ __forceinline__ T3 t3_grid(T3 a) {
+  const f2 C1 = f2_both(24.f), C2 = f2_both(0x1.8p-17f);  // units in the last place 2^-19, 2^-40
+  const f2 H = f2_sub(f2_add(a.h, C1), C1), r = f2_sub(a.h, H);
+  const f2 s = f2_add(C2, r), s2 = f2_add(s, a.m);
+  return T3{H, f2_sub(s2, C2), f2_add(f2_add(f2_sub(r, f2_sub(s, C2)), f2_sub(a.m, f2_sub(s2, s))), a.l)};
+}
+// a + c b on the grid.
+__device__ __forceinline__ T3 t3_lin(T3 a, float c, T3 b) {
+  if (c == 1.f) return T3{f2_add(a.h, b.h), f2_add(a.m, b.m), f2_add(a.l, b.l)};
+  const f2 k = f2_both(c);
+  return T3{f2_fma(b.h, k, a.h), f2_fma(b.m, k, a.m), f2_fma(b.l, k, a.l)};
+}
+__device__ __forceinline__ T3 t3_norm(T3 a) {
+  const f2 u = f2_add(a.m, a.l), v = f2_sub(a.l, f2_sub(u, a.m));
+  const f2 s = f2_add(a.h, u), e = f2_sub(u, f2_sub(s, a.h)), m = f2_add(e, v);
+  return T3{s, m, f2_sub(v, f2_sub(m, e))};
+}
+
 // K / q for q > 0 normal, K a power of two.  One Newton step makes the
 // hardware seed y accurate to half a unit, so that the residual 1 - q.h y is
 // exact; then 1 / q = y (1 + r + r^2) with r = 1 - q y, |r| < 2^-21, whose
@@ -223,24 +255,25 @@ __device__ __forceinline__ T3 t3_weno5_part(T3 q0, T3 q1, T3 q2, T3 Da, T3 Db) {
 // 6 R for both halves from the five differences d_j (WENO5); eps = 4 x the
 // reference's epsilon in the scale of d^2.  The indicators are 4 x the
 // reference's: 13/3 t^2 + s^2 + 4 eps, squared by t3_weno5_part.
-__device__ __forceinline__ T3 t3_weno5_diff(const T3 d[5], f2 eps) {
+__device__ __forceinline__ T3 t3_weno5_diff(T3 d[5], f2 eps) {
   const f2 k4 = f2_both((float)(4.0 * Lit::c13_12));  // a float exactly
-  const T3 t0 = t3_add(d[1], -1.f, d[0]), t1 = t3_add(d[2], -1.f, d[1]);
-  const T3 t2 = t3_add(d[3], -1.f, d[2]), t3 = t3_add(d[4], -1.f, d[3]);
-  const T3 sa = t3_add(d[1], 1.f, d[2]), sb = t3_add(d[2], 1.f, d[3]);
-  const T3 T1 = t3_add_f(t3_mul_f(t3_sqr(t1), k4), eps), T2 = t3_add_f(t3_mul_f(t3_sqr(t2), k4), eps);
-  const T3 D1 = t3_add(t2, -1.f, t1);
+#pragma unroll
+  for (int j = 0; j < 5; ++j) d[j] = t3_grid(d[j]);
+  auto part = [&](T3 t) { return t3_add_f(t3_mul_f(t3_sqr(t3_norm(t)), k4), eps); };
+  auto square = [&](T3 a, float c, T3 b) { return t3_sqr(t3_norm(t3_lin(a, c, b))); };
+  const T3 t0 = t3_lin(d[1], -1.f, d[0]), t1 = t3_lin(d[2], -1.f, d[1]);
+  const T3 t2 = t3_lin(d[3], -1.f, d[2]), t3 = t3_lin(d[4], -1.f, d[3]);
+  const T3 T1 = part(t1), T2 = part(t2), D1 = t3_lin(t2, -1.f, t1);
   // the difference of the two middle polynomials: d_1 - 5 d_2 - 2 d_3
-  T3 R = t3_add(t3_add(sa, -2.f, sb), -4.f, d[2]);
+  T3 R = t3_lin(t3_lin(d[1], -5.f, d[2]), -2.f, d[3]);
   {
-    const T3 T0 = t3_add_f(t3_mul_f(t3_sqr(t0), k4), eps);
-    const T3 G = t3_weno5_part(t3_add(T2, 1.f, t3_sqr(t3_add(t2, -2.f, d[2]))), t3_add(T1, 1.f, t3_sqr(sa)),
-                               t3_add(T0, 1.f, t3_sqr(t3_add(t0, 2.f, d[1]))), D1, t3_add(t1, -1.f, t0));
+    // (t2 - 2 d_2 = d_3 - 3 d_2, and t0 + 2 d_1 = -(d_0 - 3 d_1))
+    const T3 G = t3_weno5_part(t3_add(T2, 1.f, square(d[3], -3.f, d[2])), t3_add(T1, 1.f, square(d[1], 1.f, d[2])),
+                               t3_add(part(t0), 1.f, square(d[0], -3.f, d[1])), D1, t3_lin(t1, -1.f, t0));
     R = t3_add(R, -1.f, G);
   }
-  const T3 T3_ = t3_add_f(t3_mul_f(t3_sqr(t3), k4), eps);
-  const T3 G = t3_weno5_part(t3_add(T3_, 1.f, t3_sqr(t3_add(t3, -2.f, d[3]))), t3_add(T2, 1.f, t3_sqr(sb)),
-                             t3_add(T1, 1.f, t3_sqr(t3_add(t1, 2.f, d[2]))), t3_add(t3, -1.f, t2), D1);
+  const T3 G = t3_weno5_part(t3_add(part(t3), 1.f, square(d[4], -3.f, d[3])), t3_add(T2, 1.f, square(d[2], 1.f, d[3])),
+                             t3_add(T1, 1.f, square(d[1], -3.f, d[2])), t3_lin(t3, -1.f, t2), D1);
   return t3_add(R, 1.f, G);
 }
 
