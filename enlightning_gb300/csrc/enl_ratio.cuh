@@ -68,7 +68,7 @@ __device__ __forceinline__ int sensor_line(const double r[5], double ep, float e
 // the density.  Three values with the same bits are never below the threshold
 // (the ratio is ep/ep = 1 or NaN), whatever ep is: where a field is at rest,
 // which is most of a level, no FP64 operation is left.  (Eight subtractions a
-// cell were 136 us of a 4096 x 2048 level's tags; 69 now; FP32 storage 70 and 46.)
+// cell were 136 us of a 4096 x 2048 level's tags, 69 without; FP32 storage 70 and 46.)
 __device__ __forceinline__ bool tag_line64(double m, double c, double p, double ep, float epf) {
   const long long b = __double_as_longlong(c);
   if (__double_as_longlong(m) == b && __double_as_longlong(p) == b) return false;
