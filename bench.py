@@ -797,7 +797,8 @@ KERNEL_NOTES = {
               "cells under their 2x2 stencils read",
     "physbc": "physical ghost band fill (sides a stencil reads): one read and one write per band cell",
     "coarsen": "fine-to-coarse averaging: ratio^2 fine reads + one coarse write per covered coarse cell",
-    "cfl": "CFL maximum (state_scan_kernel + dt_kernel): rho, rho u, rho v of every patch cell read",
+    "cfl": "CFL maximum (state_scan_kernel + dt_kernel): rho, rho u, rho v of every patch cell read, and the "
+           "other fields and H0 where stage 1 skips uniform tiles",
 }
 
 
@@ -1114,6 +1115,9 @@ def run_linesource(args):
                                         / fp64_peak,
                                         "counting": "FP64 instructions the kernel issues (ncu: 2 per FMA, 1 per "
                                                     "add or multiply)"},
+                     "note": "the WENO reconstructions run on the FP32 pipe in three-word arithmetic, so the "
+                             "algorithmic rate passes what the FP64 pipe alone could do; implementation counts "
+                             "what that pipe issues",
                      "hbm": hbm})
     else:
         roof.update({"bound": "hbm", "achieved": hbm_achieved, "peak": hbm_peak, "unit": "GB/s",

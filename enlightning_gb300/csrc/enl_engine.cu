@@ -3332,11 +3332,11 @@ static void scan_t(Engine* E, bool records) {
 // The pass over the state at the start of a step, and the step's dt from it.
 static void scan_state(Engine* E, double dt_max, bool records) {
   if (!E->adaptive) return;
-  // rho, rho u, rho v of every patch cell (uniform tiles' other fields, read
-  // for stage 1's skipping, are not counted)
+  // rho, rho u, rho v of every patch cell, and with records the other four
+  // fields and H0
   long long cells = 0;
   for (int l = 0; l < E->cfg.nlevels; ++l) cells += E->n_cells[l];
-  const int q = kt_begin(E, 3, 3.0 * (E->f32s ? 4 : 8) * cells);
+  const int q = kt_begin(E, 3, (records ? 8.0 : 3.0) * (E->f32s ? 4 : 8) * cells);
   if (E->f32s) scan_t<float>(E, records);
   else scan_t<double>(E, records);
   dt_kernel<<<1, 1, 0, stream()>>>(E->d_smax, E->d_dt, E->d_dt + 1, reinterpret_cast<float*>(E->d_dt + 2),

@@ -3,6 +3,8 @@ enough (9,728 tiles or more) that stage 1 skips uniform tiles with its
 records: the state must be bit for bit that of the cell-by-cell computation,
 and dt the CFL rule's (one rounding each of the quotient, the sum and the
 division by the maximum: 3 x 2^-53, the storage's roundings for FP32)."""
+import ctypes as C
+
 import numpy as np
 import pytest
 
@@ -76,3 +78,40 @@ def test_dt_is_the_rule(precision):
     E.step(1.0)
     assert E.time()[0] < 1e-290
     E.close()
+
+
+@pytest.mark.parametrize("precision", [PREC_FP64, PREC_FP32_STATE])
+@pytest.mark.parametrize("learned", [False, True])
+def test_line_source_with_regrids_bit_identical(precision, learned):
+    """Three levels and regrids, stage 1 skipping all the while (10,240 base
+    tiles), with the captured step as users replay it."""
+    from enlightning_gb300 import sensor
+    out = {}
+    for dense in (True, False):
+        E, H, _ = workloads.line_source(default_params(), nx0=2048, ny0=1280, dx0=0.5, nlevels=3, nseg=60,
+                                        precision=precision, learned=learned, dense=dense)
+        if learned:
+            E.set_mlp(*sensor.load_weights())
+        E.stats()
+        torch.cuda.synchronize()
+        side = torch.cuda.Stream()  # (a capture needs a stream of its own)
+        with torch.cuda.stream(side):
+            E.L.enl_set_stream(C.c_void_p(side.cuda_stream))
+            for s in range(12):
+                if s and s % 5 == 0:
+                    H.regrid()
+                if s % 3 == 2:
+                    E.capture(1.0)
+                    E.replay(1)
+                else:
+                    E.step(1.0)
+        torch.cuda.synchronize()
+        E.L.enl_set_stream(C.c_void_p(torch.cuda.current_stream().cuda_stream))
+        torch.cuda.synchronize()
+        assert E.health() == 0
+        assert (int(E.stats()[:, 3].sum()) == 0) == dense
+        out[dense] = ([list(p) for p in E.patches], [_bits(E.buffer(l, 0)) for l in range(E.nlevels)], E.time())
+        E.close()
+    assert out[True][0] == out[False][0] and out[True][2] == out[False][2]
+    for a, b in zip(out[True][1], out[False][1]):
+        assert np.array_equal(a, b)
