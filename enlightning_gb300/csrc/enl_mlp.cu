@@ -253,29 +253,33 @@ __global__ void __launch_bounds__(128, 3) mlp_grad_kernel(const __nv_bfloat16* _
     }
     __syncthreads();
   }
-  // flush the block's partial gradients
+  // flush the block's partial gradients, two neighbouring weights an atomic (a
+  // warp's then fill their 32-byte sectors: 57.3 -> 55.8 us for 65,536 samples,
+  // 92.7 -> 90.6 for 200,000; one block of three teams an SM that sums its weight
+  // gradients in shared memory first gained no more and cost 6 us on 3,000)
+  static_assert(kOffW1 % 2 == 0 && kOffW2 % 2 == 0 && kOffB1 % 2 == 0 && kOffB2 % 2 == 0 && kHid % 2 == 0,
+                "pairs start on 8 bytes where grad does");
+  const bool pairs = (reinterpret_cast<uintptr_t>(grad) & 7) == 0;
+  auto add2 = [&](int o, float a, float b) {
+    if (pairs) {
+      atomicAdd(reinterpret_cast<float2*>(&grad[o]), make_float2(a, b));
+    } else {
+      atomicAdd(&grad[o], a);
+      atomicAdd(&grad[o + 1], b);
+    }
+  };
 #pragma unroll
   for (int n = 0; n < 8; ++n) {
     const int col = n * 8 + 2 * t;
     const int k0 = warp * 16 + g, k1 = k0 + 8;
-    atomicAdd(&grad[kOffW2 + k0 * kHid + col], aw2[n][0]);
-    atomicAdd(&grad[kOffW2 + k0 * kHid + col + 1], aw2[n][1]);
-    atomicAdd(&grad[kOffW2 + k1 * kHid + col], aw2[n][2]);
-    atomicAdd(&grad[kOffW2 + k1 * kHid + col + 1], aw2[n][3]);
+    add2(kOffW2 + k0 * kHid + col, aw2[n][0], aw2[n][1]);
+    add2(kOffW2 + k1 * kHid + col, aw2[n][2], aw2[n][3]);
     if (warp < 3) {
-      if (k0 < kFeat) {
-        atomicAdd(&grad[kOffW1 + k0 * kHid + col], aw1[n][0]);
-        atomicAdd(&grad[kOffW1 + k0 * kHid + col + 1], aw1[n][1]);
-      }
-      if (k1 < kFeat) {
-        atomicAdd(&grad[kOffW1 + k1 * kHid + col], aw1[n][2]);
-        atomicAdd(&grad[kOffW1 + k1 * kHid + col + 1], aw1[n][3]);
-      }
+      if (k0 < kFeat) add2(kOffW1 + k0 * kHid + col, aw1[n][0], aw1[n][1]);
+      if (k1 < kFeat) add2(kOffW1 + k1 * kHid + col, aw1[n][2], aw1[n][3]);
     } else if (g == 0) {  // rows 0 and 8
-      atomicAdd(&grad[kOffB1 + col], aw1[n][0]);
-      atomicAdd(&grad[kOffB1 + col + 1], aw1[n][1]);
-      atomicAdd(&grad[kOffB2 + col], aw1[n][2]);
-      atomicAdd(&grad[kOffB2 + col + 1], aw1[n][3]);
+      add2(kOffB1 + col, aw1[n][0], aw1[n][1]);
+      add2(kOffB2 + col, aw1[n][2], aw1[n][3]);
     }
 #pragma unroll
     for (int q = 0; q < 2; ++q) {
