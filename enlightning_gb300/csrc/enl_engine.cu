@@ -234,11 +234,12 @@ struct StageArgs {
   float margin;               // |p - 0.5| <= margin -> plain sensor decides
   float feat_eps, feat_eps_p, feat_inv_sqrt_eps;
   // uniform-tile skipping (null when off).  Records of the current step,
-  // per table index: stage 1 writes rec_un_out and rec_out, stage 2 writes
-  // rec_out.  In stages 2 and 3 the launch runs over a list of tiles: tiles
-  // holds their descriptors, gti their table indices (null: the table
-  // itself), and the first uniform tile computed per level is published in
-  // gcache (GUni<S>[kL]) for the skipped tiles (skip_phase).
+  // per table index: stages 1 and 2 write rec_out, and stage 1 rec_un_out
+  // where the pass at the start of the step has not.  A stage that skips runs
+  // over a list of tiles: tiles holds their descriptors, gti their table
+  // indices (null: the table itself), and the first uniform tile computed per
+  // level is published in gcache (GUni<S>[kL]) for the skipped tiles
+  // (skip_phase).
   void* rec_out;
   void* rec_un_out;
   const int* gti;

@@ -356,7 +356,7 @@ int enl_engine_profile(void* engine, int on, double* ms_total,
 /* Per-class figures of profile mode 2 since the last enl_engine_profile
  * call, six entries each: 0 coarse-fine halo interpolation, 1 physical
  * band fill, 2 coarsening, 3 CFL maximum (speed + dt kernels), and with
- * uniform-tile skipping (schedule reuse 2, RK stages 2 and 3) 4 the flag
+ * uniform-tile skipping (schedule reuse 2) 4 the flag
  * pass and tile lists, 5 the second stage launch (bytes 0 for these two;
  * their time is also inside the stage figures of enl_engine_profile).  bytes are
  * algorithmic: every cell value the launch must read or write, once
@@ -382,12 +382,15 @@ int enl_engine_set_level_order(void* engine, int samrai);
  *   sched[0] resident blocks per SM (0 = the occupancy limit),
  *   sched[1] tile order (as enl_engine_config.tile_order),
  *   sched[2] uniform-tile reuse: 2 on (the default), with RK stages 2 and 3
- *            skipping the halo box of a tile whose own and neighbours'
- *            records from the previous stage of the step prove it uniform;
+ *            (and, with adaptive dt on a large base level, stage 1) skipping
+ *            the halo box of a tile whose own and neighbours' records of the
+ *            stage's input prove it uniform;
  *            1 on, every tile's box loaded and tested; 0 off (as
  *            enl_engine_config.dense = 1),
  *   sched[3] run length: tiles a block claims at a time (1..16; consecutive
- *            tiles of a patch row, so 2 and 4 claim 64x8 and 128x8 cells).
+ *            tiles of a patch row, so 2 and 4 claim 64x8 and 128x8 cells; 1
+ *            claims an eighth of the block's share of what is left, at most 8
+ *            tiles, down to single ones).
  * Every schedule gives the same states.  Setting one invalidates a captured
  * graph.  get_schedule writes sched[0..3] (sched[0] as the actual count) and
  * sched[4] = the occupancy limit; n is the length of the array (>= 4 to set,
