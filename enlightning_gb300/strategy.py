@@ -133,19 +133,24 @@ class Enlightning:
 
     def _patch_args(self, P: Patch, absorb, ghosts):
         """The patch and the strategy's parameters as enl_patch_stage takes
-        them; filled anew by every call, so changes of either are seen."""
+        them; filled anew by every call, so changes of either are seen.
+        Vectors may have more entries than are used, as the separate entry
+        points' arguments may, and the envelope's width is read only where a
+        side absorbs."""
         p, g = self.p, P.g
         a = _lib.PatchArgs()
-        a.box[:], a.gcw[:], a.fill[:] = P.box, (g, g), (g, g)
-        a.touches[:] = [int(t) for t in P.touches]
-        a.bc[:] = self.bc if absorb else [b if b != ABSORB else 0 for b in self.bc]
+        a.box[:], a.gcw[:], a.fill[:] = list(map(int, P.box[:4])), (g, g), (g, g)
+        a.touches[:] = list(map(int, P.touches[:4]))
+        bc = self.bc[:4]
+        a.bc[:] = bc if absorb else [b if b != ABSORB else 0 for b in bc]
         a.level = int(P.level)
-        a.xlo[:], a.dx[:], a.grid_xlo[:], a.grid_xhi[:] = P.xlo, P.dx, self.domain_xlo, self.domain_xhi
-        a.tol[:] = p["tol"]
+        a.xlo[:], a.dx[:], a.tol[:] = P.xlo[:2], P.dx[:2], p["tol"][:3]
         a.weno_alpha, a.kappa, a.mu, a.muB, a.R = p["weno_alpha"], p["kappa"], p["mu"], p["muB"], p["R"]
         a.T_star_n, a.tau_n, a.c, a.c_lr, a.rho0 = p["T_star_n"], p["tau_n"], p["c"], p["c_lr"], p["rho0"]
         a.gamma1, a.c_p, a.p0, a.T0, a.c_v = p["gamma1"], p["c_p"], p["p0"], p["T0"], p["c_v"]
-        a.absorb_width = p["bc_absorb_width"]
+        if absorb and ABSORB in bc:
+            a.absorb_width = p["bc_absorb_width"]
+            a.grid_xlo[:], a.grid_xhi[:] = self.domain_xlo[:2], self.domain_xhi[:2]
         a.w_n, a.pressure, a.temperature = _ptr(P.w_scr), _ptr(P.pres), _ptr(P.temp)
         a.w, a.source, a.rhs = _ptr(P.w_cur), _ptr(P.src), _ptr(P.K)
         if ghosts:
