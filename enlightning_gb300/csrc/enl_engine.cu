@@ -1957,7 +1957,11 @@ __device__ __forceinline__ unsigned bits_of(float a) { return __float_as_uint(a)
 // operation a word.  Bound by its loads.  (With a block a tile and a thread a
 // cell, the rows' values compared through shuffles and shared memory, it was
 // bound by its instructions: 233 a warp for a row, 125 us for FP64 and 99 for
-// FP32 storage on the line source's 4096 x 2048.)
+// FP32 storage on the line source's 4096 x 2048.)  Neighbouring tiles go to
+// different blocks, and a table of at most a quarter as many tiles as the grid
+// has warps (without records) is taken by two rows: eight tiles of eight rows a
+// block left most SMs idle for four round trips to memory (640 tiles of the
+// Mach shock, FP32 storage: a step of 139.5 us before, 137.5 now).
 template <typename S, bool REC>  // blocks an SM, all resident
 constexpr int kScanBlocks = !REC ? 4 : (std::is_same<S, float>::value ? 3 : 2);
 template <typename S, bool REC>
@@ -1974,7 +1978,17 @@ __global__ void __launch_bounds__(256, kScanBlocks<S, REC>) state_scan_kernel(
   bool zero_q = false;     // FP64 storage: a cell whose speed is exactly c
   float best = 0.f;        // FP64 storage: the warp's largest quotient estimate so far
   const float roff = (float)A.rho_off, cf = (float)A.c;
-  const int step = gridDim.x * 8;
+  const int parts = !REC && 4 * n <= (int)gridDim.x * 8 ? 4 : 1;
+  const int items = n * parts, step = gridDim.x * 8;
+  auto item = [&](int e) {  // a tile, or two rows of one
+    if (e >= items) return make_int4(0, 0, 0, 0);  // w = h = 0: no cell
+    if (parts == 1) return A.tiles[e];
+    int4 d = A.tiles[e >> 2];
+    const int r0 = 2 * (e & 3), h = min(2, max(0, ((d.z >> 16) & 0xff) - r0));
+    d.y += r0;
+    d.z = (d.z & ~0xff0000) | (h << 16);
+    return d;
+  };
   auto load = [&](const int4& d, int r0, S (&x)[2][8]) {
     const int lvl = d.z & 0xff, w = (d.z >> 8) & 0xff, h = (d.z >> 16) & 0xff;
     if (lane >= w) return;
@@ -1994,13 +2008,12 @@ __global__ void __launch_bounds__(256, kScanBlocks<S, REC>) state_scan_kernel(
       }
     }
   };
-  const int4 none = make_int4(0, 0, 0, 0);  // w = h = 0: no cell
-  int t = blockIdx.x * 8 + warp;
-  int4 td = t < n ? A.tiles[t] : none, nd = t + step < n ? A.tiles[t + step] : none;
+  int t = warp * gridDim.x + blockIdx.x;
+  int4 td = item(t), nd = item(t + step);
   S buf[2][2][8];
   load(td, 0, buf[0]);
-  for (; t < n; t += step) {
-    const int4 d2 = t + 2 * step < n ? A.tiles[t + 2 * step] : none;
+  for (; t < items; t += step) {
+    const int4 d2 = item(t + 2 * step);
     const int w = (td.z >> 8) & 0xff, h = (td.z >> 16) & 0xff;
     U first[8], acc = 0;
     float est[8], top = best;
