@@ -229,10 +229,18 @@ __device__ __forceinline__ void split_speeds64(const SAcc64P<TH>& A, const RhsCo
 // + cx) holds the nw WENO cells of a mixed tile; without it every cell of the
 // w x h tile is one.  j0 is the index of the tile's first row for the height
 // of the split speeds.  D[p * 32 TH + cell] receives the flux part -(dF/dx +
-// dG/dy) of field p or, with one or two rows, -dF/dx of field p < 5 and -dG/dy
-// of field p - 5.
+// dG/dy) of field p or, with one or two rows, the unscaled differences along x
+// of field p < 5 and along y of field p - 5, which weno_part64 scales and adds
+// with the same operations: a cell's result does not depend on the size of its
+// patch.
 template <int TH>
 constexpr int kFluxParts64 = TH <= 2 ? 10 : 5;
+// -(dF/dx + dG/dy) from weno_flux64's differences (rounded as written: the
+// compiler must not fuse the last product into the caller's sum).
+template <int ORDER>
+__device__ __forceinline__ double weno_scaled64(const RhsConst& P, double dfx, double dgy) {
+  return __dmul_rn(ORDER == 5 ? Lit::c1_6 : 0.5, fma(dfx, P.inv_dx0, __dmul_rn(dgy, P.inv_dx1)));
+}
 template <int ORDER, bool LLF, int TH>
 __device__ __forceinline__ void weno_tasks64(const double* tile, const double* pl, const RhsConst& P, int j0, int w,
                                              int h, const int* list, int nw, double* D) {
@@ -240,7 +248,6 @@ __device__ __forceinline__ void weno_tasks64(const double* tile, const double* p
   constexpr int kParts = kFluxParts64<TH>;
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
   const int nchunk = list ? (nw + 31) >> 5 : h;
-  const double c = ORDER == 5 ? Lit::c1_6 : 0.5;
   for (int t = warp; t < kParts * nchunk; t += 8) {
     const int part = t / nchunk, q = t - part * nchunk;
     int cell;
@@ -263,19 +270,20 @@ __device__ __forceinline__ void weno_tasks64(const double* tile, const double* p
     if constexpr (kParts == 5) {
       const double dfx = weno_flux64<ORDER>(wk, 1, fk, 1, ha);
       const double dgy = weno_flux64<ORDER>(wk, kBW64, gk, 32, hb);
-      d = fma(dfx, P.inv_dx0, dgy * P.inv_dx1);
+      d = weno_scaled64<ORDER>(P, dfx, dgy);
     } else {
       const bool y = part >= 5;
-      d = weno_flux64<ORDER>(wk, y ? kBW64 : 1, y ? gk : fk, y ? 32 : 1, y ? hb : ha) * (y ? P.inv_dx1 : P.inv_dx0);
+      d = weno_flux64<ORDER>(wk, y ? kBW64 : 1, y ? gk : fk, y ? 32 : 1, y ? hb : ha);
     }
-    D[part * (32 * TH) + cell] = c * d;
+    D[part * (32 * TH) + cell] = d;
   }
 }
 // -(dF/dx + dG/dy) of field k of a WENO cell from weno_tasks64's parts.
-template <int TH>
-__device__ __forceinline__ double weno_part64(const double* D, int cell, int k) {
-  if constexpr (kFluxParts64<TH> == 5) return D[k * (32 * TH) + cell];
-  else return D[k * (32 * TH) + cell] + D[(k + 5) * (32 * TH) + cell];
+template <int ORDER, int TH>
+__device__ __forceinline__ double weno_part64(const double* D, const RhsConst& P, int cell, int k) {
+  const double d = D[k * (32 * TH) + cell];
+  if constexpr (kFluxParts64<TH> == 5) return d;
+  else return weno_scaled64<ORDER>(P, d, D[(k + 5) * (32 * TH) + cell]);
 }
 
 // Accessor of the learned switch's features on an FP64 tile: density and

@@ -94,7 +94,7 @@ __global__ void __launch_bounds__(256, 2)
   sources64(A, P, H);
   if (flag) {
 #pragma unroll
-    for (int k = 0; k < 5; ++k) H[k] += weno_part64<TH>(flux, tid, k);
+    for (int k = 0; k < 5; ++k) H[k] += weno_part64<ORDER, TH>(flux, P, tid, k);
   } else {
     drp_flux64(A, P, H);
   }
