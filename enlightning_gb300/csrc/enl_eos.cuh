@@ -332,9 +332,13 @@ inline EosConst64 make_eos_const64(double rho0, double c, double c_lr, double ga
                     (R / c_v) * std::fma(-rho0, 1.0 / rho0, 1.0)};
 }
 
-// Any density and entropy (zero, negative, non-finite, far from ambient).
-static __device__ __noinline__ double temperature_general64(const EosConst64& E, double w0, double w3) {
-  return E.T0 * exp((w3 / w0 - E.R * log(E.rho0 / w0)) / E.c_v);
+// Any density and entropy (zero, negative, non-finite, far from ambient): .x the
+// temperature; .y the pressure's term rho / c_p (rho s / rho) where it is not
+// finite (a zero or infinite density, an entropy per mass beyond the range),
+// which the sum of eos64 without that quotient has to take on, else 0.
+static __device__ __noinline__ double2 state_general64(const EosConst64& E, double w0, double w3) {
+  const double s = w3 / w0, q = w0 * E.inv_c_p * s;
+  return double2{E.T0 * exp((s - E.R * log(E.rho0 / w0)) / E.c_v), isfinite(q) ? 0.0 : q};
 }
 
 // p and T of a cell; height = centre height of the cell row.  Every operation
@@ -365,7 +369,9 @@ __device__ __forceinline__ void eos64(const EosConst64& E, double w0, double w3,
       return;
     }
   }
-  T = temperature_general64(E, w0, w3);
+  const double2 g = state_general64(E, w0, w3);
+  T = g.x;
+  p = __dadd_rn(p, g.y);
 }
 
 }  // namespace enl
