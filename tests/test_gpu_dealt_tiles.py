@@ -1,8 +1,9 @@
 """The stage kernel's deal: every block's first run of tiles, and its second
 where runs are single tiles, come from the block's index, the rest from the
-counter.  Tables around one, two and sixteen tiles a block, in each tile order
-and run length, give the state of the schedule that counts every tile (order 3)
-bit for bit; and a table of fewer tiles than blocks takes one tile's time."""
+counter (in FP64, up to eight tiles a block, when the tile before is done).
+Tables around one, two, eight and sixteen tiles a block, in each tile order and
+run length, give the state of the schedule that counts every tile (order 3) bit
+for bit; and a table of fewer tiles than blocks takes one tile's time."""
 import numpy as np
 import pytest
 
@@ -30,7 +31,7 @@ def row_of_tiles(n, precision, variant="hybrid_high_llf"):
 
 
 @pytest.mark.parametrize("precision", [PREC_FP64, PREC_FP32_STATE])
-@pytest.mark.parametrize("share", [0, 1, 2, 16])
+@pytest.mark.parametrize("share", [0, 1, 2, 8, 16])
 def test_every_tile_once(precision, share):
     nsm = torch.cuda.get_device_properties(0).multi_processor_count
     for n in sorted({max(1, share * nsm + d) for d in (-1, 0, 1)}):
