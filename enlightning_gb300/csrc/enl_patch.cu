@@ -104,33 +104,19 @@ __global__ void __launch_bounds__(256, 2)
 }
 
 // runge_kutta.m4:60-63, association kept: (a1*ww + a2*w_n) + (beta*dt)*KK.
-// Bound by memory: blockIdx.z takes one field, and a thread has the loads of
-// kRkCells cells (32 columns apart) in flight at once.
-constexpr int kRkCells = 4;
-__global__ void __launch_bounds__(128) runge_kutta_kernel(double* __restrict__ wn, long pitch, long fstride, int g0,
-                                                          int g1, const double* __restrict__ ww,
-                                                          const double* __restrict__ KK, long ipitch, long ifstride,
-                                                          int nx, int ny, double a1, double a2, double bdt) {
-  const int ci = blockIdx.x * (32 * kRkCells) + threadIdx.x, cj = blockIdx.y * blockDim.y + threadIdx.y;
-  if (cj >= ny) return;
-  double* wr = wn + blockIdx.z * fstride + (long)(cj + g1) * pitch + g0;
-  const double* ur = ww + blockIdx.z * ifstride + (long)cj * ipitch;
-  const double* kr = KK + blockIdx.z * ifstride + (long)cj * ipitch;
-  double u[kRkCells], w[kRkCells], k[kRkCells];
-#pragma unroll
-  for (int q = 0; q < kRkCells; ++q) {
-    const int i = ci + 32 * q;
-    if (i < nx) {
-      u[q] = ur[i];
-      w[q] = wr[i];
-      k[q] = kr[i];
-    }
-  }
-#pragma unroll
-  for (int q = 0; q < kRkCells; ++q) {
-    const int i = ci + 32 * q;
-    if (i < nx) wr[i] = __dadd_rn(__dadd_rn(__dmul_rn(a1, u[q]), __dmul_rn(a2, w[q])), __dmul_rn(bdt, k[q]));
-  }
+// A thread takes a cell of all fields: bound by launching on a small patch and
+// by memory on a large one.  (A thread with four cells of one field in flight
+// did the same on 512 x 512, 16.6 us, and less well where its blocks are many
+// for their cells: 16 x 5000 12.4 and 26.8 us, 300 x 217 7.0 and 8.0.)
+__global__ void runge_kutta_kernel(double* __restrict__ wn, long pitch, long fstride, int g0, int g1,
+                                   const double* __restrict__ ww, const double* __restrict__ KK, long ipitch,
+                                   long ifstride, int nx, int ny, int nequ, double a1, double a2, double bdt) {
+  const int ci = blockIdx.x * blockDim.x + threadIdx.x, cj = blockIdx.y * blockDim.y + threadIdx.y;
+  if (ci >= nx || cj >= ny) return;
+  const long g = (long)(cj + g1) * pitch + (ci + g0), c = (long)cj * ipitch + ci;
+  for (int k = 0; k < nequ; ++k)
+    wn[k * fstride + g] = __dadd_rn(__dadd_rn(__dmul_rn(a1, ww[k * ifstride + c]), __dmul_rn(a2, wn[k * fstride + g])),
+                                    __dmul_rn(bdt, KK[k * ifstride + c]));
 }
 
 // update_state.m4:87-107 (eos64).
@@ -405,21 +391,22 @@ __global__ void __launch_bounds__(256) update_kernel(const __grid_constant__ Upd
 
 // The same walks serially, for a patch that lies partly outside the domain
 // (its distance from a side is not positive at the walk's first cell, so the
-// factors need not grow along the walk): one thread per row or column.
-__global__ void absorb_walk_kernel(PatchFields8 F, long pitch, int nx, int ny, int g0, int g1, int dir,
-                                   AbsorbConst A) {
+// factors need not grow along the walk): one thread per row or column, and one
+// kernel per side, since what depends on the side lies on the walk's chain (64 x
+// 64 cells, four sides: 873 us with the side as an argument, 728 so).
+template <int DIR>
+__global__ void absorb_walk_kernel(PatchFields8 F, long pitch, int nx, int ny, int g0, int g1, AbsorbConst A) {
   const double ep = 1.0e-8;
-  const int t = blockIdx.x * blockDim.x + threadIdx.x;
-  const bool x = dir < 2;
+  constexpr bool x = DIR < 2, upper = DIR & 1;
+  const int t = blockIdx.x * blockDim.x + threadIdx.x, len = x ? nx : ny;
   if (t >= (x ? ny : nx)) return;
-  const int len = x ? nx : ny;
   auto dist = [&](int c) {
     const double q = x ? A.xlo0 + A.dx0 * ((double)c + 0.5) : A.xlo1 + A.dx1 * ((double)c + 0.5);
-    return (dir & 1) ? ((x ? A.gxhi0 : A.gxhi1) - q) : (q - (x ? A.gxlo0 : A.gxlo1));
+    return upper ? ((x ? A.gxhi0 : A.gxhi1) - q) : (q - (x ? A.gxlo0 : A.gxlo1));
   };
-  double tmp = (!x || t == 0) ? envelope(dist((dir & 1) ? len - 1 : 0), A.w2) : 0.0;
+  double tmp = (!x || t == 0) ? envelope(dist(upper ? len - 1 : 0), A.w2) : 0.0;
   for (int n = 0; (fabs(1.0 - tmp) > ep) && n < len; ++n) {
-    const int c = (dir & 1) ? len - 1 - n : n;
+    const int c = upper ? len - 1 - n : n;
     tmp = envelope(dist(c), A.w2);
     absorb_apply(F, x ? (long)(t + g1) * pitch + (c + g0) : (long)(c + g1) * pitch + (t + g0), tmp, A);
   }
@@ -624,9 +611,10 @@ void runge_kutta_(const int& ifirst0, const int& ilast0, const int& ifirst1, con
     return;
   }
   long pitch = nx + 2 * gcw0, fstride = pitch * (ny + 2 * gcw1);
-  const dim3 block(32, 4), grid((nx + 32 * kRkCells - 1) / (32 * kRkCells), (ny + 3) / 4, nequ);
-  runge_kutta_kernel<<<grid, block, 0, stream()>>>(w_n, pitch, fstride, gcw0, gcw1, w, rhs, nx, (long)nx * ny, nx, ny,
-                                                   alpha_1, alpha_2, beta * dt);
+  const dim3 block(32, 4);
+  runge_kutta_kernel<<<grid2d(nx, ny, block), block, 0, stream()>>>(w_n, pitch, fstride, gcw0, gcw1, w, rhs, nx,
+                                                                    (long)nx * ny, nx, ny, nequ, alpha_1, alpha_2,
+                                                                    beta * dt);
   check_launch("runge_kutta");
 }
 
@@ -739,10 +727,14 @@ int enl_absorb(int ifirst0, int ilast0, int ifirst1, int ilast1, int gcw0, int g
   if (inside) {
     absorb_kernel<<<dim3((nx + 31) / 32, (ny + 7) / 8), 256, 0, stream()>>>(F, pitch, nx, ny, gcw0, gcw1, dirs, A);
   } else {
-    for (int dir = 0; dir < 4; ++dir)
+    auto walk = [&](auto kernel, int dir) {
       if (dirs & (1 << dir))
-        absorb_walk_kernel<<<((dir < 2 ? ny : nx) + 127) / 128, 128, 0, stream()>>>(F, pitch, nx, ny, gcw0, gcw1, dir,
-                                                                                    A);
+        kernel<<<((dir < 2 ? ny : nx) + 127) / 128, 128, 0, stream()>>>(F, pitch, nx, ny, gcw0, gcw1, A);
+    };
+    walk(absorb_walk_kernel<0>, 0);
+    walk(absorb_walk_kernel<1>, 1);
+    walk(absorb_walk_kernel<2>, 2);
+    walk(absorb_walk_kernel<3>, 3);
   }
   return check_launch("absorb");
 }
