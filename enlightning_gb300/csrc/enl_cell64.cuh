@@ -230,7 +230,7 @@ __device__ __forceinline__ void split_speeds64(const SAcc64P<TH>& A, const RhsCo
 // w x h tile is one.  j0 is the index of the tile's first row for the height
 // of the split speeds.  D[p * 32 TH + cell] receives the flux part -(dF/dx +
 // dG/dy) of field p or, with one or two rows, the unscaled differences along x
-// of field p < 5 and along y of field p - 5, which weno_part64 scales and adds
+// of field p < 5 and along y of field p - 5, which weno_join64 scales and adds
 // with the same operations: a cell's result does not depend on the size of its
 // patch.
 template <int TH>
@@ -278,12 +278,18 @@ __device__ __forceinline__ void weno_tasks64(const double* tile, const double* p
     D[part * (32 * TH) + cell] = d;
   }
 }
-// -(dF/dx + dG/dy) of field k of a WENO cell from weno_tasks64's parts.
+// After weno_tasks64 and a barrier: leaves the flux part of field k of a cell
+// in D[k * 32 TH + cell], by the whole block of 256 threads, with a barrier
+// where there is something to join.  (Joined by the cells' own threads, one or
+// two warps of the eight, 24 x 16 cells took 18.6 us, so 16.8.  What it makes
+// of cells that are not WENO cells is not read.)
 template <int ORDER, int TH>
-__device__ __forceinline__ double weno_part64(const double* D, const RhsConst& P, int cell, int k) {
-  const double d = D[k * (32 * TH) + cell];
-  if constexpr (kFluxParts64<TH> == 5) return d;
-  else return weno_scaled64<ORDER>(P, d, D[(k + 5) * (32 * TH) + cell]);
+__device__ __forceinline__ void weno_join64(double* D, const RhsConst& P) {
+  if constexpr (kFluxParts64<TH> == 10) {
+    constexpr int n = 5 * 32 * TH;
+    for (int e = threadIdx.x; e < n; e += 256) D[e] = weno_scaled64<ORDER>(P, D[e], D[e + n]);
+    __syncthreads();
+  }
 }
 
 // Accessor of the learned switch's features on an FP64 tile: density and

@@ -1157,7 +1157,7 @@ __global__ void __launch_bounds__(256, std::is_same<S, float>::value ? kStageBlo
             sources64(acc, A.P[lvl], K);
             if (f) {
 #pragma unroll
-              for (int k = 0; k < 5; ++k) K[k] += weno_part64<ORDER, kTH>(flux64, A.P[lvl], tid, k);
+              for (int k = 0; k < 5; ++k) K[k] += flux64[k * (32 * kTH) + tid];
             } else {
               drp_flux64(acc, A.P[lvl], K);
             }

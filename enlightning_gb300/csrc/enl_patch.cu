@@ -85,6 +85,7 @@ __global__ void __launch_bounds__(256, 2)
     }
     weno_tasks64<ORDER, LLF, TH>(tile, pl, P, j0, tw, th, all ? nullptr : s_list, nw, flux);
     __syncthreads();
+    weno_join64<ORDER, TH>(flux, P);
   }
   if (!valid) return;
   const SAcc64P<TH> A = acc64p<TH>(tile, pl, lane, warp);
@@ -94,7 +95,7 @@ __global__ void __launch_bounds__(256, 2)
   sources64(A, P, H);
   if (flag) {
 #pragma unroll
-    for (int k = 0; k < 5; ++k) H[k] += weno_part64<ORDER, TH>(flux, P, tid, k);
+    for (int k = 0; k < 5; ++k) H[k] += flux[k * (32 * TH) + tid];
   } else {
     drp_flux64(A, P, H);
   }
