@@ -655,8 +655,8 @@ __global__ void __launch_bounds__(256, std::is_same<S, float>::value ? kStageBlo
   __shared__ __align__(16) int4 s_dq;  // descriptor and table index on their way (thread 0)
   __shared__ int s_gq;
   __shared__ int s_run;    // end of the block's run of claimed tiles (thread 0)
-  constexpr bool kLate = !FAST;  // (claims)
-  __shared__ int s_late;   // the next tile is claimed after this one (thread 0)
+  constexpr bool kLate = !FAST && SCHEME == kHybrid;  // (claims)
+  __shared__ int s_late;   // the next tile is claimed after this one
   __shared__ int s_next;   // the block's second tile where it is dealt out, else -1 (thread 0)
   __shared__ int s_dealt;  // tiles dealt out; the counter counts from there (thread 0)
   __shared__ UniEntry<S> s_uc[kL];
@@ -684,13 +684,13 @@ __global__ void __launch_bounds__(256, std::is_same<S, float>::value ? kStageBlo
   // with the first tile dealt and 139 with two (the second round backwards,
   // the last blocks first: 148); tables of thousands of tiles the same within
   // 0.3 %.
-  // With the FP64 right-hand side, whose tiles differ (20 us and 100) by more
+  // With the hybrid scheme in FP64, whose tiles differ (20 us and 100) by more
   // than a box's way to shared memory takes, a table of at most two tiles a
   // block is claimed late, the second tile when the first is done: 484 tiles on
-  // 304 blocks 432 us from the counter ahead, 467 dealt, 384 late; 538 455, 425
-  // and 366; but 800 alike 904, 903 and 919, 1,600 1,566, 1,565 and 1,594 (and
-  // FP32 tiles take 9 us: 5,596 on 608 blocks 247 dealt, 255 late).  Orders 2
-  // and 3, which mix the table's ends as the blocks arrive, count every tile
+  // 304 blocks 432 us from the counter ahead, 467 dealt, 386 late; 538 455, 425
+  // and 370.  (800 tiles alike 904, 903 and 919; 484 of WENO alone 865, 868 and
+  // 877; FP32 tiles take 9 us: 5,596 on 608 blocks 247 dealt, 255 late.)  Orders
+  // 2 and 3, which mix the table's ends as the blocks arrive, count every tile
   // (order 2, line source of 2048 x 1024: 1,016 us a step, 1,043 dealt).
   auto claim = [&](int cur) -> int {
     if (A.tile_order == 3) {
@@ -795,15 +795,27 @@ __global__ void __launch_bounds__(256, std::is_same<S, float>::value ? kStageBlo
   uint32_t phase[2] = {0u, 0u};
   int b = 0;
   int t = s_t[0];
-  auto advance = [&]() {  // claims the next tile and issues its copies (thread 0)
-    const bool ahead = t + 1 < s_run;  // its descriptor is on its way
-    int nt = claim(t);
-    if (!ahead) fetch(nt);
-    if (nt < ntiles && !issue(nt, b ^ 1)) nt = ntiles;
-    s_t[b ^ 1] = nt;
-  };
+  // the next tile is claimed and its copies issued when a tile starts; a late
+  // block takes turns, a tile and then the claim
+  const bool late = kLate && s_late;
+  bool turn = !late;
   while (t < ntiles) {
-    if (tid == 0 && !(kLate && s_late)) advance();
+    if (tid == 0 && turn) {
+      const bool ahead = t + 1 < s_run;  // its descriptor is on its way
+      int nt = claim(t);
+      if (!ahead) fetch(nt);
+      if (nt < ntiles && !issue(nt, b ^ 1)) nt = ntiles;
+      s_t[b ^ 1] = nt;
+    }
+    if (kLate && late) {
+      turn = !turn;
+      if (!turn) {
+        __syncthreads();
+        t = s_t[b ^ 1];
+        b ^= 1;
+        continue;
+      }
+    }
     const double* tile = reinterpret_cast<const double*>(dst[b]);  // FP64 storage
     float* tile32 = kF32S ? reinterpret_cast<float*>(dst[b]) : tile32_conv;
     const int4 td = s_td[b];
@@ -1208,8 +1220,8 @@ __global__ void __launch_bounds__(256, std::is_same<S, float>::value ? kStageBlo
         }
       }
     }
-    if (kLate && tid == 0 && s_late) advance();
     __syncthreads();  // this staging buffer is refilled two tiles later
+    if (kLate && late) continue;
     t = s_t[b ^ 1];
     b ^= 1;
   }
