@@ -134,7 +134,7 @@ __device__ __forceinline__ int switch64(const SAcc64P<TH>& A, const RhsConst& P)
 //   rho / T A_n M_n - rho / T_n c_vn M_n = -rho c_vn M_n / T.
 // What remains is (viscous heating + kappa lap T - c_vn H4) / T with H4 = rho
 // M_n.  The differences stay unscaled and the viscosities, the grid spacings
-// and the literals 4/3 and 2/3 are in the launch constants (visc_const); the
+// and the literals 4/3 and 2/3 are in the launch constants (make_rhs_const); the
 // heating muB (u_x + v_y)^2 + mu/2 (phi_xx^2 + 2 phi_xy^2 + phi_yy^2) is the
 // quadratic form qa (u_x^2 + v_y^2) + qb u_x v_y + mu phi_xy^2.  As the
 // reference writes it the sources took 122 operations.

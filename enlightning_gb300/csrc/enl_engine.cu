@@ -228,7 +228,6 @@ struct StageArgs {
   unsigned long long* stats;  // [level][4]: weno cells, cells, cells decided by the plain-sensor fallback,
                               // cells of uniform tiles stored from the cache
   AbsorbTables absorb;        // absorbing envelope, applied to each finished cell
-  bool any_absorb;
   const int4* patchtab;       // patch boxes of all levels (tile .w = index)
   const MlpSmem* mlp;         // learned-sensor network image (global memory) or null
   float margin;               // |p - 0.5| <= margin -> plain sensor decides
@@ -260,20 +259,6 @@ struct StageArgs {
 };
 
 // Shared-memory accessors centred on one cell of the staged halo tile.
-struct SAcc64 {
-  const double* t;  // tile base
-  int c;            // (row)*kBW + col of the centre
-  __device__ double w(int k, int di, int dj) const { return t[k * (kBH * kBW) + c + dj * kBW + di]; }
-  __device__ double p(int di, int dj) const { return t[5 * (kBH * kBW) + c + dj * kBW + di]; }
-  __device__ double t_(int di, int dj) const { return t[6 * (kBH * kBW) + c + dj * kBW + di]; }
-  __device__ double tT(int di, int dj) const { return t_(di, dj); }
-};
-struct SAcc64R {  // adapter with the accessor names rhs_cell expects
-  SAcc64 a;
-  __device__ double w(int k, int di, int dj) const { return a.w(k, di, dj); }
-  __device__ double p(int di, int dj) const { return a.p(di, dj); }
-  __device__ double t(int di, int dj) const { return a.tT(di, dj); }
-};
 struct SAcc32 {  // single-precision tile and its planes
   const float* t;
   const float* pl;  // u, v, F_0..4, G_0..4
@@ -2944,12 +2929,15 @@ static int rebuild_tables(Engine* E) {
   // A table whose tiles repay stage 1's skipping: uniform tiles are the base
   // level's (finer levels lie where the waves are).  On the 33,000 base tiles of
   // the line source's 4096 x 2048, most of them uniform, a step takes 3.56 ms
-  // without and 3.31 with it (FP64), 0.744 and 0.638 (FP32 storage): 8 and 3 ns
-  // a tile, against 28 and 15 us for the records, flags, lists and second
-  // launch (the Mach shock, 2,048 base and 7,680 fine tiles, few of them
-  // uniform, in FP64: 9.560 and 9.587 ms).  Hence on from 16 base tiles a block
-  // of a full grid (4,864 and 9,728), off below half of that: a captured step
-  // does not change with every new table.
+  // without and 3.31 with it (FP64), 0.744 and 0.638 (FP32 storage).  Smaller
+  // line sources, us without and with it:
+  //   base tiles   3,200          4,608          6,272          8,192          12,800
+  //   FP64         1,255 1,274    1,440 1,413    1,600 1,604    1,752 1,723    2,143 2,079
+  //   FP32           279   288      297   296      320   323      350   341      431   408
+  // and the Mach shock (2,048 base and 7,680 fine tiles, few of them uniform)
+  // 9,019 and 9,042, 1,269 and 1,291.  Hence on from 16 base tiles a block of a
+  // full grid (4,864 and 9,728), off below half of that: a captured step does
+  // not change with every new table.
   {
     const int most = 16 * E->nsm * E->max_blocks_per_sm;
     const bool many = nl > 0 && E->tile_cnt[0] >= (E->many_tiles ? most / 2 : most);
@@ -3123,7 +3111,6 @@ static StageArgs stage_args(Engine* E, int stage, double dt, int level = -1) {
   A.betaf = (float)A.beta;
   A.bdtf = (float)A.bdt;
   A.absorb = absorb_tables(E);
-  A.any_absorb = any_absorb(E);
   A.patchtab = E->d_patchtab.p;
   A.tiles = E->d_tiles.p;
   A.ntiles = E->d_meta + (level < 0 ? M_NTILES : M_TILE_CNT + level);
@@ -3440,9 +3427,11 @@ static void record_mics(Engine* E) {
 }
 
 // RK stage `stage` with skipping: flags and lists from the records of its
-// input (stage 0: the scan's, in stage 1's output records' place), the launch over the tiles to compute (its blocks then
-// store the skipped tiles, skip_phase), and a launch over the skipped tiles
-// without a cached or published result (usually none).
+// input (stage 0: the scan's, in the place of stage 2's outputs), the launch
+// over the tiles to compute (its blocks then store the skipped tiles,
+// skip_phase), and a launch over the skipped tiles without a cached or
+// published result (usually none; all of them on a table so small that no
+// block has a result yet when the skipped tiles are taken).
 template <typename S>
 static void skip_stage_t(Engine* E, int stage, StageFn fn, const StageArgs& A0) {
   cudaStream_t s = stream();

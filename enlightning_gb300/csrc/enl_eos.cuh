@@ -15,9 +15,9 @@
 namespace enl {
 
 // Table of the logarithm: the mantissa range [0.707, 1.414) in 256 steps of the
-// high word; c is near the reciprocal of the step's middle (exactly 1 on both
-// sides of 1, so that log is accurate where its value is small) and the second
-// entry is -log(c).
+// high word; c is the double next to the reciprocal of the step's middle
+// (exactly 1 on both sides of 1, so that log is accurate where its value is
+// small) and the second entry the double next to -log(c).
 __device__ const double2 kLogTable64[256] = {
     {0x1.6993f349cc726p+0, -0x1.61965cdb02c1ep-2}, {0x1.68954dd2390bap+0, -0x1.5ec433d5c35aep-2},
     {0x1.67980e0bf08c7p+0, -0x1.5bf406b543db1p-2}, {0x1.669c31075ab40p+0, -0x1.5925d2b112a59p-2},

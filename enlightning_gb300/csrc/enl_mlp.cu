@@ -24,14 +24,16 @@ namespace enl {
 //   * Every fragment comes from shared memory by ldmatrix (four 8 x 8 tiles per
 //     instruction, transposed where the product runs over samples) from
 //     conflict-free padded rows; W2 is kept once, its transpose read from it.
-//   * GELU and its derivative are evaluated together, once per activation.
+//   * GELU and its derivative are evaluated once per activation, not once more
+//     where the derivative is needed.
 //   * Bias gradients are a product with a row of ones on the tensor cores,
 //     done by the warp that has no rows of dW1, and dw3 is accumulated in
 //     registers; one warp summing 64 samples column by column kept the other
 //     three waiting.
 //   * As many blocks as fit (no second wave that stages the parameters again),
 //     features read 16 bytes at a time.
-// 65,536 samples: 84 -> 53 us a call (with its two clears).
+// 65,536 samples: 84 -> 53 us a call among others (with its two clears; a call
+// alone 86 -> 54).
 // ---------------------------------------------------------------------------
 constexpr int kChunk = 64;
 
@@ -49,8 +51,9 @@ static_assert(offsetof(MlpSmem, w1t) % 16 == 0 && offsetof(MlpSmem, w2t) % 16 ==
                   offsetof(TrainSmem, dz2) % 16 == 0 && kLdF * 2 % 16 == 0 && kLdH * 2 % 16 == 0,
               "16-byte rows");
 
-// GELU and its derivative: Phi(x) by erf_as, whose exponential is the
-// density's, exp(-x^2 / 2).
+// GELU and its derivative at one argument, in one place so that the compiler
+// shares Phi(x) between them (erf_as's exponential and the density's round their
+// arguments differently and stay two).
 __device__ __forceinline__ void gelu_both(float x, float& g, float& d) {
   g = gelu(x);
   d = gelu_grad(x);
@@ -254,8 +257,8 @@ __global__ void __launch_bounds__(128, 3) mlp_grad_kernel(const __nv_bfloat16* _
     __syncthreads();
   }
   // flush the block's partial gradients, two neighbouring weights an atomic (a
-  // warp's then fill their 32-byte sectors: 57.3 -> 55.8 us for 65,536 samples,
-  // 92.7 -> 90.6 for 200,000; one block of three teams an SM that sums its weight
+  // warp's then fill their 32-byte sectors: a call alone 57.3 -> 55.8 us for 65,536
+  // samples, 92.7 -> 90.6 for 200,000; one block of three teams an SM that sums its weight
   // gradients in shared memory first gained no more and cost 6 us on 3,000)
   static_assert(kOffW1 % 2 == 0 && kOffW2 % 2 == 0 && kOffB1 % 2 == 0 && kOffB2 % 2 == 0 && kHid % 2 == 0,
                 "pairs start on 8 bytes where grad does");

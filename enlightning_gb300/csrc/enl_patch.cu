@@ -30,9 +30,9 @@ int rhs_variant();
 // field (weno_tasks64), and every thread finishes one cell.  The arithmetic is
 // the batched engine's (enl_cell64.cuh).  Bound by the FP64 and FP32 pipes.
 // One thread per cell reading the patch through L1, with 23 FP64 divisions and
-// 40 FP64 reconstructions a WENO cell, took 430 us on 512x512 (hybrid, level
-// 0), 129 us on 131x93 (fine level) and 111 us on 24x16; this takes 171, 35
-// and 25 us.
+// 40 FP64 reconstructions a WENO cell, took 444 us on 512x512 (hybrid, level
+// 0), 111 us on 131x93 (fine level) and 118 us on 24x16 (level 0); this takes
+// 113, 33 and 21 us.
 //
 // TH: 8 rows for large patches (the least work for the halo: 14 rows of
 // planes for 8 of cells); fewer rows when the patch has too few tiles for the
@@ -466,12 +466,18 @@ RhsConst make_rhs_const(const double* xlo, const double* dx, double alpha, doubl
 // work for its halo (TH + 6 rows of planes for TH of cells).  Two blocks run on
 // an SM.  Measured, hybrid scheme on level 0 / on a fine level (WENO in every
 // cell), us for 8, 4, 2, 1 rows:
-//   32x32    73 43 29 25    / 66 38 25 19
-//   131x93   76 44 42 52    / 66 39 35 48
-//   256x256  87 76 74 113   / 105 109 111 146
-//   384x384  130 108 127 213 / 202 206 236 312
-//   512x512  179 171 205 351 / 336 334 390 534
-//   700x700  280 299 356 617 / 588 592 704 983
+//   32x32    62 38 25 21    / 58 35 23 17
+//   131x93   66 40 39 46    / 59 35 33 42
+//   256x256  69 59 59 85    / 93 99 101 132
+//   384x384  97 78 89 154   / 175 184 211 278
+//   512x512  129 113 144 257 / 289 300 349 477
+//   700x700  181 202 247 462 / 506 535 629 883
+// the lower-order hybrid scheme and DRP alone:
+//   32x32    42 27 20 17    / 19 12 11 11
+//   131x93   47 29 29 35    / 19 12 13 15
+//   256x256  52 48 51 77    / 31 31 37 48
+//   512x512  115 113 143 251 / 97 97 113 155
+//   700x700  179 203 257 461 / 171 175 207 284
 // so 8 rows from four waves of blocks on, 4 from one wave, 2 from half a wave.
 static int rhs_rows(int nx, int ny) {
   const long cols = (nx + 31) / 32;

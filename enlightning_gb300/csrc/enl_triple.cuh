@@ -34,11 +34,13 @@
 // difference, so with the differences d_j = x_{j+1} - x_j, t_j = d_{j+1} -
 // d_j and D_j = t_{j+1} - t_j
 //   6 wenop(lo) = f1 - w0 D_1 - 2 w2 D_0,
-// and R needs nothing but differences: constant parts cancel before the
-// first rounding.  The routine therefore takes the differences of F/2 and w
-// in FP64, forms d_j for both signs (10 fused multiply-adds) and converts
-// them exactly, scaled by the largest one's power of two, so that no value of
-// the state overflows or underflows the single-precision range.
+// and R needs nothing but differences.  The routine therefore takes the
+// differences of F/2 and w in FP64 (F/2 is a rounded half flux, and a
+// difference is rounded unless the two lie within a factor of two of each
+// other), forms d_j for both signs (10 fused multiply-adds, rounded) and
+// converts those to three words, scaled by the largest one's power of two, so
+// that no value of the state overflows or underflows the single-precision
+// range: exactly, down to 2^-75 of the largest.
 #pragma once
 #include "enl_rcp.cuh"
 

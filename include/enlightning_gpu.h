@@ -355,7 +355,7 @@ int enl_engine_profile(void* engine, int on, double* ms_total,
 
 /* Per-class figures of profile mode 2 since the last enl_engine_profile
  * call, six entries each: 0 coarse-fine halo interpolation, 1 physical
- * band fill, 2 coarsening, 3 CFL maximum (speed + dt kernels), and with
+ * band fill, 2 coarsening, 3 CFL maximum (state scan + dt kernels), and with
  * uniform-tile skipping (schedule reuse 2) 4 the flag
  * pass and tile lists, 5 the second stage launch (bytes 0 for these two;
  * their time is also inside the stage figures of enl_engine_profile).  bytes are
