@@ -390,7 +390,8 @@ int enl_engine_set_level_order(void* engine, int samrai);
  *   sched[3] run length: tiles a block claims at a time (1..16; consecutive
  *            tiles of a patch row, so 2 and 4 claim 64x8 and 128x8 cells; 1
  *            claims an eighth of the block's share of what is left, at most 8
- *            tiles, down to single ones).
+ *            tiles, down to single ones; in tile orders 0 and 1 a block's
+ *            first tiles come from its index).
  * Every schedule gives the same states.  Setting one invalidates a captured
  * graph.  get_schedule writes sched[0..3] (sched[0] as the actual count) and
  * sched[4] = the occupancy limit; n is the length of the array (>= 4 to set,
